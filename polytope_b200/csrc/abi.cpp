@@ -54,10 +54,41 @@ int upload(void** dst, const T* src, size_t count, uint64_t& bytes) {
     return PT_OK;
 }
 
+// The four-wide records of the scene's tree, made on the device from the uploaded nodes.  A tree with
+// a box outside its parent's (only a caller's own tree can have one) or of extreme size gets none and
+// keeps the binary walk, as does one whose records do not fit in memory.
+int make_wide(pt_scene* s, const HostScene& h) {
+    if (h.wide_of.empty() || s->nan_boxes) return PT_OK;
+    const size_t n = h.wide_of.size();
+    for (int k = 0; k < 3; ++k)
+        s->wide_size = std::max(s->wide_size, std::max(std::fabs(h.nodes[0].bb_min[k]), std::fabs(h.nodes[0].bb_max[k])));
+    if (!(s->wide_size >= kWideSizeMin && s->wide_size <= kWideSizeMax)) return PT_OK;
+    // behind the records: the numbering and the flag, in the same allocation (scene creation waits for
+    // each cudaMalloc, now and then for milliseconds)
+    const size_t record_bytes = 64 * (size_t)h.num_wide;
+    if (cudaMalloc(&s->dev.wide, record_bytes + 4 * (n + 1)) != cudaSuccess) {
+        cudaGetLastError();
+        s->dev.wide = nullptr;
+        return PT_OK;
+    }
+    uint32_t* tmp = (uint32_t*)((char*)s->dev.wide + record_bytes);
+    uint32_t outside = 0;
+    cudaError_t e = cudaMemcpy(tmp, h.wide_of.data(), 4 * n, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemset(tmp + n, 0, 4);
+    if (e == cudaSuccess) e = launch_wide_make(s->dev.nodes, tmp, (uint32_t)n, s->wide_size, 0, s->dev.wide, s->dev.tris, tmp + n, nullptr);
+    if (e == cudaSuccess) e = cudaMemcpy(&outside, tmp + n, 4, cudaMemcpyDeviceToHost);
+    if (e != cudaSuccess) return cuda_fail(e, "four-wide records");
+    if (outside) {
+        cudaFree(s->dev.wide);
+        s->dev.wide = nullptr;
+    }
+    return PT_OK;
+}
+
 void free_scene(pt_scene* s) {
     if (!s) return;
     DeviceGuard g(s->device);
-    void* bufs[] = {s->dev.nodes, s->dev.tris, s->dev.meshes, s->dev.prim_normals, s->dev.prim_tri,
+    void* bufs[] = {s->dev.nodes, s->dev.tris, s->dev.wide, s->dev.meshes, s->dev.prim_normals, s->dev.prim_tri,
                     s->dev.light_tris, s->dev.light_cdf, s->dev.instances, s->dev.tlas_nodes, s->dev_in, s->dev_out,
                     s->err_flag, s->trace_err, s->ray_counters};
     for (void* b : bufs)
@@ -129,6 +160,8 @@ int scene_trace(pt_scene* s, const pt_ray* rays, uint64_t n, pt_hit* hits, uint3
     a.top_nodes = s->dev.tlas_nodes;
     a.top_num_nodes = s->dev.tlas_num_nodes;
     a.exact_tree = s->nan_boxes;
+    a.wide = s->dev.wide;
+    a.wide_size = s->wide_size;
     auto next_counter = [s]() {
         return (void*)((unsigned long long*)s->ray_counters + (s->counter_next.fetch_add(1) % PT_RAY_COUNTERS));
     };
@@ -276,7 +309,7 @@ int prepare_scene_host(const pt_scene_desc* desc, HostScene& h) {
         rc = build_bvh(desc->meshes, desc->num_meshes, w, 0, t);
         if (rc) return rc;
     }
-    rc = validate_tree(t.nodes.data(), (uint32_t)t.nodes.size(), w.num_prims, &h.max_depth);
+    rc = validate_tree(t.nodes.data(), (uint32_t)t.nodes.size(), w.num_prims, &h.max_depth, &h.wide_of, &h.num_wide);
     if (rc) return rc;
     h.num_prims = w.num_prims;
     h.prim_base = w.prim_base;
@@ -421,6 +454,7 @@ int create_from_host(const pt_scene_desc* desc, HostScene& h, pt_scene** out) {
         return false;
     };
     s->nan_boxes = has_nan(h.nodes) || has_nan(h.tlas);
+    if ((rc = make_wide(s.get(), h))) { free_scene(s.release()); return rc; }
     if (h.two_level) {
         s->two_level = true;
         s->dev.num_instances = (uint32_t)h.instances.size();

@@ -437,18 +437,22 @@ int build_bvh(const pt_mesh_desc* meshes, uint32_t num_meshes, const WorldMeshes
     return PT_OK;
 }
 
-int validate_tree(const pt_bvh_node* nodes, uint32_t num_nodes, uint32_t num_leaf_entries, uint32_t* max_depth_out) {
+int validate_tree(const pt_bvh_node* nodes, uint32_t num_nodes, uint32_t num_leaf_entries, uint32_t* max_depth_out,
+                  std::vector<uint32_t>* wide_of, uint32_t* num_wide) {
     if (num_nodes == 0) return fail(PT_EINVAL, "empty tree");
     std::vector<uint32_t> depth(num_nodes, 0);
     std::vector<uint8_t> seen(num_nodes, 0);
     seen[0] = 1;
-    uint32_t max_depth = 0;
+    uint32_t max_depth = 0, records = 0;
+    bool shared = false;  // a node with two parents: no record numbering by depth
+    if (wide_of) wide_of->assign(num_nodes, kNotWide);
     // Pre-order layout: every child index is larger than its parent's, so one forward sweep
     // visits parents first.
     for (uint32_t i = 0; i < num_nodes; ++i) {
         if (!seen[i]) continue;
         const pt_bvh_node& n = nodes[i];
         max_depth = std::max(max_depth, depth[i]);
+        if (wide_of && (i == 0 || (n.num_faces == 0 && (depth[i] & 1u) == 0))) (*wide_of)[i] = records++;
         if (n.num_faces > 0) {
             if ((uint64_t)n.offset + n.num_faces > num_leaf_entries)
                 return fail(PT_EINVAL, "leaf " + std::to_string(i) + " face range out of bounds");
@@ -458,10 +462,16 @@ int validate_tree(const pt_bvh_node* nodes, uint32_t num_nodes, uint32_t num_lea
         const uint64_t lo = (uint64_t)i + 1, hi = (uint64_t)i + n.offset;
         if (n.offset < 2 || hi >= num_nodes || lo >= num_nodes)
             return fail(PT_EINVAL, "node " + std::to_string(i) + ": child index out of bounds");
+        shared = shared || seen[lo] || seen[hi];
         seen[lo] = seen[hi] = 1;
         depth[lo] = depth[hi] = depth[i] + 1;
     }
     if (max_depth_out) *max_depth_out = max_depth;
+    if (wide_of && (shared || num_nodes > (1u << 28))) {
+        wide_of->clear();
+        records = 0;
+    }
+    if (num_wide) *num_wide = records;
     return PT_OK;
 }
 

@@ -25,7 +25,15 @@ struct TraceArgs {
     const void* top_nodes = nullptr;
     uint32_t top_num_nodes = 0;
     bool exact_tree = false;  // some box holds a NaN: every ray takes the exact box test
+    const void* wide = nullptr;  // four-wide records (wide.cuh), or null: the binary walk
+    float wide_size = 0.f;       // largest coordinate of the tree's boxes
 };
+
+// Four-wide records of the tree of num_nodes nodes at `nodes` (faces from face_base of `tris`, whose last
+// words receive their leaf's node).  wide_of: the record that starts at each node, ~0 for none.
+// *outside is set when some box does not lie inside its parent's, or some face inside its leaf's.
+cudaError_t launch_wide_make(const void* nodes, const uint32_t* wide_of, uint32_t num_nodes, float size, uint32_t face_base,
+                             void* wide, void* tris, uint32_t* outside, cudaStream_t s);
 
 cudaError_t launch_trace(const TraceArgs& a, cudaStream_t s);
 

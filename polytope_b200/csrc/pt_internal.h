@@ -65,7 +65,13 @@ int scene_trace(pt_scene* s, const pt_ray* rays, uint64_t n, pt_hit* hits, uint3
                 uint32_t* tri_tests, uint32_t mem_flags, void* stream);
 
 // Checks that every child / leaf range stays inside the arrays and computes the deepest level.
-int validate_tree(const pt_bvh_node* nodes, uint32_t num_nodes, uint32_t num_leaf_entries, uint32_t* max_depth);
+// wide_of (optional) receives the number of the four-wide record (wide.cuh) that starts at each
+// node, kNotWide where none does, and num_wide their count: the root and the interior nodes at even
+// depth.  Empty when some node has two parents (a caller's own tree) or the indices do not fit.
+constexpr uint32_t kNotWide = 0xFFFFFFFFu;
+constexpr float kWideSizeMin = 9.3132257e-10f, kWideSizeMax = 1.0737418e9f;  // 2^-30, 2^30: the trees wide.cuh is proved for
+int validate_tree(const pt_bvh_node* nodes, uint32_t num_nodes, uint32_t num_leaf_entries, uint32_t* max_depth,
+                  std::vector<uint32_t>* wide_of = nullptr, uint32_t* num_wide = nullptr);
 
 // ---- device scene -------------------------------------------------------------------------------
 struct DeviceMesh {  // per-mesh shading record (device)
@@ -87,6 +93,8 @@ struct HostScene {  // host copy of everything a scene handle uploads
     uint32_t num_prims = 0;
     uint32_t max_depth = 0;
     std::vector<uint32_t> prim_base;
+    std::vector<uint32_t> wide_of;    // four-wide record that starts at each node (empty: none are made)
+    uint32_t num_wide = 0;
     // two-level layout (pt_scene_create_two_level): `nodes` / `tris` then hold every distinct
     // geometry's object-space tree and faces back to back, and these the instances and the top
     // level over their world boxes
@@ -107,6 +115,7 @@ struct SceneDev {
     // traversal data
     void* nodes = nullptr;        // num_nodes * 32 B  (pt_bvh_node)
     void* tris = nullptr;         // num_prims * 48 B  (3 x float4 per leaf-ordered entry)
+    void* wide = nullptr;         // four-wide records of the tree (wide.cuh), 64 B each, or null
     // shading data
     void* meshes = nullptr;       // num_meshes * DeviceMesh
     void* prim_normals = nullptr; // num_prims * 9 floats (world vertex normals by prim id) or null
@@ -151,6 +160,7 @@ struct pt_scene {
     void* err_flag = nullptr;
     void* trace_err = nullptr;
     bool two_level = false;  // made by pt_scene_create_two_level
+    float wide_size = 0.f;   // largest coordinate of the tree's boxes (wide.cuh)
     bool nan_boxes = false;  // some tree box holds a NaN (every ray then takes the exact box test)
     // ray counters of the persistent trace kernel: one per launch in flight, taken round-robin
     void* ray_counters = nullptr;

@@ -4,11 +4,13 @@
 // HBM once (32 B in, 16 B out per ray); nodes and faces are read with 128-bit read-only loads and
 // stay resident in the 126 MB L2 for scenes up to a few million faces.
 
+#include <algorithm>
 #include <type_traits>
 
 #include "launch.h"
 #include "traverse.cuh"
 #include "two_level.cuh"
+#include "wide.cuh"
 
 namespace pt {
 
@@ -162,6 +164,125 @@ __global__ void __launch_bounds__(128, 8) trace_persistent_kernel(const uint4* _
     }
 }
 
+// ---- four-wide walk ---------------------------------------------------------------------------------
+
+__global__ void __launch_bounds__(128) wide_make_kernel(const uint4* __restrict__ nodes, const uint32_t* __restrict__ wide_of,
+                                                        uint32_t num_nodes, float size, uint32_t face_base, WideNode* __restrict__ wide,
+                                                        float4* __restrict__ tris, uint32_t* outside) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= num_nodes) return;
+    bool ok = true;
+    if ((nodes[2 * (size_t)i + 1].w & 0xFFFFu) != 0) ok = wide_mark_leaf(nodes, i, face_base, tris);
+    if (wide_of[i] != 0xFFFFFFFFu) {
+        WideNode w;
+        ok = wide_make(nodes, wide_of, i, size, w) && ok;
+        const uint4* src = (const uint4*)&w;
+        uint4* dst = (uint4*)(wide + wide_of[i]);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) dst[k] = src[k];
+    }
+    if (!ok) atomicExch(outside, 1u);
+}
+
+cudaError_t launch_wide_make(const void* nodes, const uint32_t* wide_of, uint32_t num_nodes, float size, uint32_t face_base,
+                             void* wide, void* tris, uint32_t* outside, cudaStream_t s) {
+    if (!num_nodes) return cudaSuccess;
+    wide_make_kernel<<<(num_nodes + 127) / 128, 128, 0, s>>>((const uint4*)nodes, wide_of, num_nodes, size, face_base,
+                                                             (WideNode*)wide, (float4*)tris, outside);
+    return cudaGetLastError();
+}
+
+// Ray queries over the four-wide records, persistent as above.  A lane's state is what its walk meets
+// next (WideWalkT::cur): records are visited together until PT_WIDE_BATCH lanes hold a leaf (or all that
+// still walk), then those test their faces together; lanes whose ray has ended wait until PT_WIDE_REFILL
+// of them store their hits and take new rays together.  A batch smaller than the resident warps spreads
+// over all of them, a few rays a warp, and needs neither counter nor memset.
+template <int SH>
+__global__ void __launch_bounds__(128, PT_WIDE_BLOCKS) trace_wide_kernel(const WideNode* __restrict__ wide, const uint4* __restrict__ nodes,
+                                                            const float4* __restrict__ tris, uint32_t num_nodes,
+                                                            const float4* __restrict__ rays, uint4* __restrict__ hits, uint32_t n,
+                                                            int* err, unsigned long long* counter, uint32_t chunk, float size) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t warp = blockIdx.x * 4 + (threadIdx.x >> 5);
+    // this warp's rays: first its own chunk, then those that the counter hands out (base + chunk <= n + 2^12)
+    uint32_t pool_next = warp * chunk < n ? warp * chunk : n, pool_end = n - pool_next < chunk ? n : pool_next + chunk;
+    bool exhausted = false, loaded = false;  // loaded: the lane holds a ray whose hit is not yet stored
+    uint32_t idx = 0;
+    __shared__ uint2 sstack[SH > 0 ? SH * 128 : 1];
+    WideWalkT<kWideStack, SH> k;
+    k.stack.base = sstack + threadIdx.x;
+    k.stack.stride = 128;
+    k.cur = kWideDone;
+    k.binary = false;
+    auto dir = [&](float& x, float& y, float& z) {
+        const float4 d = rays[2 * (size_t)idx + 1];
+        x = d.x; y = d.y; z = d.z;
+    };
+    while (true) {
+        // lanes whose ray has ended store its hit and take the next ray, PT_WIDE_REFILL at a time
+        const uint32_t ended = __ballot_sync(0xFFFFFFFFu, k.cur == kWideDone);
+        if (__popc(ended) >= (exhausted ? 32 : PT_WIDE_REFILL)) {
+            if (k.cur == kWideDone && loaded) {
+                bool ok = !k.done || k.any || k.binary;
+                uint4 h;
+                if (k.binary) {
+                    const float4 r0 = rays[2 * (size_t)idx], r1 = rays[2 * (size_t)idx + 1];
+                    const BinaryRay ray{r0.x, r0.y, r0.z, r1.x, r1.y, r1.z, r0.w, k.any};
+                    BinaryHit b;
+                    ok = wide_binary_walk(nodes, tris, num_nodes, &ray, &b);
+                    h = make_uint4(b.prim, __float_as_uint(b.t), __float_as_uint(b.u), __float_as_uint(b.v));
+                } else {
+                    h = make_uint4(k.prim, __float_as_uint(k.min_t), __float_as_uint(k.u), __float_as_uint(k.v));
+                }
+                if (!ok) {
+                    h.x = 0xFFFFFFFEu;
+                    atomicExch(err, 1);
+                }
+                st_stream(hits + idx, h);
+                loaded = false;
+            }
+            if (!exhausted && pool_next >= pool_end) {
+                unsigned long long base = (unsigned long long)gridDim.x * 4 * chunk;
+                if (base < n) {
+                    if (lane == 0) base += atomicAdd(counter, (unsigned long long)chunk);
+                    base = __shfl_sync(0xFFFFFFFFu, base, 0);
+                }
+                if (base >= n) {
+                    exhausted = true;
+                } else {
+                    pool_next = (uint32_t)base;
+                    pool_end = n - pool_next < chunk ? n : pool_next + chunk;
+                }
+            }
+            const uint32_t avail = pool_end - pool_next;
+            const uint32_t rank = __popc(ended & ((1u << lane) - 1u));
+            if (k.cur == kWideDone && rank < avail) {
+                idx = pool_next + rank;
+                const float4 r0 = ld_stream(rays + 2 * (size_t)idx);
+                const float4 r1 = ld_stream(rays + 2 * (size_t)idx + 1);
+                wide_begin(k, r0.x, r0.y, r0.z, r1.x, r1.y, r1.z, r0.w, (__float_as_uint(r1.w) & 1u) != 0, size);
+                loaded = true;
+            }
+            const uint32_t took = min((uint32_t)__popc(ended), avail);
+            pool_next += took;
+            if (took == 0 && exhausted && ended == 0xFFFFFFFFu) break;
+            continue;
+        }
+        const bool at_leaf = k.cur != kWideDone && (k.cur & kWideLeaf);
+        const uint32_t leaves = __ballot_sync(0xFFFFFFFFu, at_leaf);
+        const uint32_t live = __popc(~ended);
+        if (__popc(leaves) >= (live < PT_WIDE_BATCH ? live : PT_WIDE_BATCH)) {
+            if (at_leaf) {
+                wide_faces(k, tris, nodes, dir);
+                if (k.done) k.cur = kWideDone; else wide_pop(k);
+            }
+        } else if (k.cur != kWideDone && !at_leaf) {
+            if (wide_visit(k, wide)) wide_pop(k);
+            else { k.done = true; k.any = k.binary = false; k.cur = kWideDone; }  // guard failure
+        }
+    }
+}
+
 // Ray queries on a two-level scene: one thread per ray, traverse_two_level.
 template <bool COUNT>
 __global__ void __launch_bounds__(128) trace_two_level_kernel(const TwoLevelView v, const float4* __restrict__ rays,
@@ -210,6 +331,22 @@ cudaError_t launch_trace(const TraceArgs& a, cudaStream_t s) {
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         const bool counted = a.node_tests || a.tri_tests;
         const int sh = a.shared_stack;
+        if (a.wide && !counted && a.n < 0xFFFF0000ull) {  // 32-bit ray numbers
+            auto kern = sh >= 32 ? trace_wide_kernel<32> : sh >= 24 ? trace_wide_kernel<24> : sh >= 16 ? trace_wide_kernel<16>
+                        : sh >= 8 ? trace_wide_kernel<8> : trace_wide_kernel<0>;
+            cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 128, 0);
+            if (e != cudaSuccess) return e;
+            const uint64_t warps = (uint64_t)sms * (per_sm < 1 ? 1 : per_sm) * 4;
+            uint64_t ch = a.chunk ? a.chunk : 64u;
+            ch = std::max<uint64_t>(1, std::min(ch, (a.n + warps - 1) / warps));
+            const uint64_t grid = std::min<uint64_t>(warps / 4, ((a.n + ch - 1) / ch + 3) / 4);
+            if (grid * 4 * ch < a.n) e = cudaMemsetAsync(a.counter, 0, sizeof(unsigned long long), s);
+            if (e != cudaSuccess) return e;
+            kern<<<(unsigned)grid, 128, 0, s>>>((const WideNode*)a.wide, (const uint4*)a.nodes, (const float4*)a.tris, a.num_nodes,
+                                                (const float4*)a.rays, (uint4*)a.hits, (uint32_t)a.n, a.err, (unsigned long long*)a.counter,
+                                                (uint32_t)ch, a.wide_size);
+            return cudaGetLastError();
+        }
         auto pick = [sh](auto k0, auto k8, auto k16, auto k24, auto k32) {
             return sh >= 32 ? k32 : sh >= 24 ? k24 : sh >= 16 ? k16 : sh >= 8 ? k8 : k0;
         };
