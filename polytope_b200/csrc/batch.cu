@@ -251,6 +251,8 @@ int wf_build(pt_batch* b, const pt_batch_item* items, const pt_batch_tuning& t) 
     b->wt.stack_cap = b->cap;
     b->wt.paths = t.pipeline == PT_PIPELINE_PATHS;
     b->wt.two_level = b->two_level;
+    b->wt.wide = true;
+    for (const pt_scene* sc : b->scenes) b->wt.wide = b->wt.wide && sc->dev.wide;
     return PT_OK;
 }
 

@@ -41,11 +41,12 @@
 #define PT_PATH_MIN_BLOCKS 7
 #endif
 
-// Ray queries over four-wide records (trace_wide_kernel): resident blocks of 128 threads a SM, lanes at a
-// leaf before faces are tested, ended lanes before new rays are taken.  Measured on a B200 (us, 16.7 M
-// rays on 1.3 M faces / 1 M rays on 100 k box faces / 1 M occlusion rays on 330 k faces): 5 blocks (96
-// registers, no spills) 5443 / 465 / 575, 6 (80 registers) 5753 / 486 / 611, 7 6089 / 527 / 649, 8 6759 /
-// 595 / 724; leaf batch 12 with refill 4 at 5 blocks 5786 / 475 / 566.
+// Walks over four-wide records: resident blocks of 128 threads a SM, lanes at a leaf before faces are
+// tested, ended lanes before new rays are taken, and visits a lane makes between votes.  Measured on a
+// B200 (us; 16.7 M rays on 1.3 M faces / 1 M rays on 100 k box faces / 1 M occlusion rays on 330 k
+// faces): 4 visits 5190 / 427 / 562, 1: 5450 / 464 / 578, 2: 5357 / 438 / 568, 8: 5387 / 438 / 605; at 4
+// visits, 6 blocks (80 registers, spills) 5484 / 437 / 586, 4 blocks 5696 / 447 / 552; leaf batch 12
+// 5280 / 427 / 554, 20 5328 / 441 / 590.
 #ifndef PT_WIDE_BLOCKS
 #define PT_WIDE_BLOCKS 5
 #endif
@@ -54,4 +55,29 @@
 #endif
 #ifndef PT_WIDE_REFILL
 #define PT_WIDE_REFILL 8
+#endif
+#ifndef PT_WIDE_STEPS
+#define PT_WIDE_STEPS 4
+#endif
+
+// The same for the persistent path kernel (wf_wide_path_kernel), with the lanes that must have a ray to
+// end or start, or a hit to shade, before those steps run.  Measured on a B200 (ms; 1920x1080x16 frame
+// of 3.9 M faces / 641x479x4 frame of 20 k box faces / 24 served requests), before the binary walk's
+// kernel and after: 12.9 / 3.35 / 9.0 -> 9.4 / 2.7 / 6.1.  One visit between votes 9.5 / 3.0 / 6.5; 4 blocks
+// 10.2 / 2.85 / 6.2, 6 blocks 9.4 / 2.7 / 6.1 (one visit: 11.1 / 3.3 / 7.1); turns from 4 or 16 lanes on
+// within 2 %, shading from 10 or 24 lanes on 3 to 7 % slower on the first.
+#ifndef PT_WIDE_PATH_BLOCKS
+#define PT_WIDE_PATH_BLOCKS 5
+#endif
+#ifndef PT_WIDE_BATCH_PATHS
+#define PT_WIDE_BATCH_PATHS 12
+#endif
+#ifndef PT_WIDE_TURNS
+#define PT_WIDE_TURNS 8
+#endif
+#ifndef PT_WIDE_SHADES
+#define PT_WIDE_SHADES 16
+#endif
+#ifndef PT_WIDE_PATH_STEPS
+#define PT_WIDE_PATH_STEPS 4
 #endif

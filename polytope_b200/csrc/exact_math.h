@@ -126,8 +126,16 @@ PT_HD void raise_flag(int* flag) {
     *flag = 1;
 #endif
 }
-PT_HD float next_up(float x) { return nextafterf(x, bitsf(0x7F800000u)); }
-PT_HD float next_down(float x) { return nextafterf(x, bitsf(0xFF800000u)); }
+// The next number above (below) x: one step of the bit pattern, away from zero or towards it.  NaN and
+// the infinity on that side stay; from zero the first subnormal.  The same values as nextafterf, whose
+// twelve inlined copies were a tenth of the shading code.
+PT_HD float next_toward(float x, bool up) {
+    const uint32_t b = fbits(x), mag = b & 0x7FFFFFFFu;
+    const bool away = (b >> 31 == 0) == up;
+    if (mag == 0) return bitsf(up ? 1u : 0x80000001u);
+    if (mag > 0x7F800000u || (mag == 0x7F800000u && away)) return x;
+    return bitsf(away ? b + 1 : b - 1);
+}
 
 // constants.h:62,142-148: gamma_n = (n * eps) / (1 - n * eps) with eps = 2^-24, in float, and
 // BoundingBox.cpp:27: 1 + 2 * Gamma(3).  Bit patterns (checked against the host compiler's
@@ -309,7 +317,12 @@ float f64_diff_emulated(float a, float b, float c, float d) {
 // ------------------------------------------------------------------------------------------------
 // Counter-based RNG: Philox4x32-10 (Salmon, Moraes, Dror, Shaw, SC'11).
 PT_HD void philox4x32(uint32_t c[4], uint32_t k0, uint32_t k1) {
-#pragma unroll
+#ifdef PT_PHILOX_UNROLL
+    constexpr int kUnroll = PT_PHILOX_UNROLL;
+#else
+    constexpr int kUnroll = 10;
+#endif
+#pragma unroll kUnroll
     for (int r = 0; r < 10; ++r) {
         const uint64_t p0 = (uint64_t)0xD2511F53u * c[0];
         const uint64_t p1 = (uint64_t)0xCD9E8D57u * c[2];

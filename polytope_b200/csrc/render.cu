@@ -204,6 +204,8 @@ RenderParams render_params(const pt_scene* s, const pt_render_desc* desc) {
     p.top_nodes = s->dev.tlas_nodes;
     p.top_num_nodes = s->dev.tlas_num_nodes;
     p.exact_tree = s->nan_boxes ? 1u : 0u;
+    p.wide = s->dev.wide;
+    p.wide_size = s->wide_size;
     return p;
 }
 
@@ -305,6 +307,7 @@ int enqueue_frame(pt_scene* s, const pt_render_desc* desc, float* rgb_d, uint32_
         t.stack_cap = stack_cap_for(s->max_depth, 0);
         t.paths = persistent;
         t.two_level = s->two_level;
+        t.wide = s->dev.wide != nullptr;
         // paths a warp takes per fetch: large chunks cost fewer fetches on a large frame (128
         // measured best on the 6.5 M-face 1920x1080x64 frame: 1771 Msamples/s against 1721 at 64,
         // 1751 at 256, 1660 at 512), while a frame too small to give every resident warp 16

@@ -42,6 +42,8 @@ struct RenderParams {
     const void* top_nodes;
     uint32_t top_num_nodes;
     uint32_t exact_tree;  // some tree box holds a NaN: every ray takes the exact box test
+    float wide_size;      // four-wide records (wide.cuh) and the tree's largest coordinate; null: the binary walk
+    const void* wide;
 };
 
 // Paths [first, first + count) in sample-major order (path p = sample * W*H + pixel).

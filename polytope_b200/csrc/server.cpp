@@ -318,7 +318,11 @@ cudaError_t pt_server::enqueue(WaveInFlight& w, const std::vector<uint32_t>& tak
         wt.queue_chunk = cfg.tuning.queue_chunk;
         wt.stack_cap = cap;
         wt.paths = cfg.tuning.pipeline == PT_PIPELINE_PATHS;
-        for (Request* r : w.members) wt.two_level = wt.two_level || r->scene->two_level;
+        wt.wide = true;
+        for (Request* r : w.members) {
+            wt.two_level = wt.two_level || r->scene->two_level;
+            wt.wide = wt.wide && r->scene->dev.wide;
+        }
         char* dt = (char*)d_tables;
         if (e == cudaSuccess)
             e = pt::wf_launch_wave((const pt::WfItem*)dt, (const pt::WfSegment*)(dt + ib), (const pt::WfPixels*)(dt + ib + sb),

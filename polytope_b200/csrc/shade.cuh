@@ -86,9 +86,9 @@ PT_HD HitFrame hit_frame(F3 v0, F3 v1, F3 v2, float u, float v, float w, F3 d,
     F3 off = vscale(n, dd);
     if (vdot(d, n) > 0) off = {-off.x, -off.y, -off.z};
     F3 np = vadd(loc, off);
-    if (off.x > 0) np.x = next_up(np.x); else if (off.x < 0) np.x = next_down(np.x);
-    if (off.y > 0) np.y = next_up(np.y); else if (off.y < 0) np.y = next_down(np.y);
-    if (off.z > 0) np.z = next_up(np.z); else if (off.z < 0) np.z = next_down(np.z);
+    if (off.x > 0 || off.x < 0) np.x = next_toward(np.x, off.x > 0);
+    if (off.y > 0 || off.y < 0) np.y = next_toward(np.y, off.y > 0);
+    if (off.z > 0 || off.z < 0) np.z = next_toward(np.z, off.z > 0);
     const float d0 = fabs_(vdot(e0, e1)), d1 = fabs_(vdot(e1, e2)), d2 = fabs_(vdot(e2, e0));
     F3 t1;
     if (d0 > d1 && d0 > d2) t1 = e0;

@@ -273,12 +273,15 @@ __global__ void __launch_bounds__(128, PT_WIDE_BLOCKS) trace_wide_kernel(const W
         const uint32_t live = __popc(~ended);
         if (__popc(leaves) >= (live < PT_WIDE_BATCH ? live : PT_WIDE_BATCH)) {
             if (at_leaf) {
-                wide_faces(k, tris, nodes, dir);
+                wide_faces(k, tris, [&]() { return nodes; }, dir);
                 if (k.done) k.cur = kWideDone; else wide_pop(k);
             }
-        } else if (k.cur != kWideDone && !at_leaf) {
-            if (wide_visit(k, wide)) wide_pop(k);
-            else { k.done = true; k.any = k.binary = false; k.cur = kWideDone; }  // guard failure
+        } else {
+#pragma unroll 1
+            for (int step = 0; step < PT_WIDE_STEPS && !(k.cur & kWideLeaf); ++step) {
+                if (wide_visit(k, wide)) wide_pop(k);
+                else { k.done = true; k.any = k.binary = false; k.cur = kWideDone; }  // guard failure
+            }
         }
     }
 }

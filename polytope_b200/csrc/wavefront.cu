@@ -1,9 +1,11 @@
 // wavefront.cu -- the multi-render wavefront engine (see wavefront.h).
 
 #include <algorithm>
+#include <type_traits>
 
 #include "path.cuh"
 #include "wavefront.h"
+#include "wide.cuh"
 
 namespace pt {
 
@@ -187,6 +189,124 @@ __global__ void __launch_bounds__(256, kWfTraceMinBlocks) wf_trace_kernel(const 
     }
 }
 
+// The same over four-wide records (every item has them; see trace_wide_kernel): visits until
+// PT_WIDE_BATCH lanes hold a leaf, then faces; ended lanes store their results and take queue entries
+// PT_WIDE_REFILL at a time.
+template <bool SHADOW, int THREADS>
+__global__ void __launch_bounds__(THREADS, 128 * PT_WIDE_BLOCKS / THREADS) wf_wide_kernel(const WfItem* __restrict__ items, WfState ws,
+                                                       const uint32_t* __restrict__ queue, const uint32_t* count_ptr,
+                                                       unsigned long long* fetch, uint32_t chunk,
+                                                       unsigned long long* rays_traced) {
+    constexpr int SH = 16;
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t n = *count_ptr;
+    uint32_t pool_next = 0, pool_end = 0, slot = 0, entry = 0, rays = 0;
+    bool exhausted = false, loaded = false;  // loaded: the lane holds a ray whose result is not yet stored
+    const WideNode* wide = nullptr;
+    const float4* tris = nullptr;
+    const RenderParams* p = nullptr;
+    __shared__ uint2 sstack[SH * THREADS];
+    WideWalkT<kWideStack, SH> k;
+    k.stack.base = sstack + threadIdx.x;
+    k.stack.stride = THREADS;
+    k.cur = kWideDone;
+    auto dir = [&](float& x, float& y, float& z) {
+        const float4 d = SHADOW ? ws.sh_d[entry] : ws.ray_d[slot];
+        x = d.x; y = d.y; z = d.z;
+    };
+    while (true) {
+        const uint32_t ended = __ballot_sync(0xFFFFFFFFu, k.cur == kWideDone);
+        if (__popc(ended) >= (exhausted ? 32 : PT_WIDE_REFILL)) {
+            if (k.cur == kWideDone && loaded) {
+                bool ok = !k.done || k.any || k.binary;
+                if (k.binary) {
+                    const float4 o4 = SHADOW ? ws.sh_o[entry] : ws.ray_o[slot];
+                    float dx, dy, dz;
+                    dir(dx, dy, dz);
+                    const BinaryRay ray{o4.x, o4.y, o4.z, dx, dy, dz, SHADOW ? o4.w : __int_as_float(0x7F800000), k.any};
+                    BinaryHit b;
+                    ok = wide_binary_walk((const uint4*)p->nodes, (const float4*)p->tris, p->num_nodes, &ray, &b);
+                    k.prim = b.prim; k.leaf = b.leaf;
+                    k.u = b.u; k.v = b.v; k.w = b.w;
+                }
+                if (!ok) atomicExch(p->err, 1);
+                if (SHADOW) {
+                    if (ok && k.prim == kPrimNone) {  // one shadow ray per slot per bounce: no other writer
+                        const float4 c = ws.sh_c[entry];
+                        float4 l = ws.rad[slot];
+                        l.x = fadd(l.x, c.x);
+                        l.y = fadd(l.y, c.y);
+                        l.z = fadd(l.z, c.z);
+                        ws.rad[slot] = l;
+                    }
+                } else {
+                    ws.hit[slot] = make_uint4(ok ? k.prim : kPrimNone, k.leaf, __float_as_uint(k.u), __float_as_uint(k.v));
+                    ws.hit_w[slot] = k.w;
+                }
+                loaded = false;
+            }
+            if (!exhausted && pool_next >= pool_end) {
+                unsigned long long base = 0;
+                if (lane == 0) base = atomicAdd(fetch, (unsigned long long)chunk);
+                base = __shfl_sync(0xFFFFFFFFu, base, 0);
+                if (base >= n) {
+                    exhausted = true;
+                } else {
+                    pool_next = (uint32_t)base;
+                    pool_end = n - pool_next < chunk ? n : pool_next + chunk;
+                }
+            }
+            const uint32_t avail = pool_end - pool_next;
+            const uint32_t rank = __popc(ended & ((1u << lane) - 1u));
+            if (k.cur == kWideDone && rank < avail) {
+                entry = pool_next + rank;
+                float4 o4, d4;
+                float tmax;
+                if (SHADOW) {
+                    o4 = ws.sh_o[entry];
+                    d4 = ws.sh_d[entry];
+                    slot = __float_as_uint(d4.w);
+                    tmax = o4.w;
+                } else {
+                    slot = queue[entry];
+                    o4 = ws.ray_o[slot];
+                    d4 = ws.ray_d[slot];
+                    tmax = __int_as_float(0x7F800000);
+                }
+                p = items[__float_as_uint(SHADOW ? ws.ray_o[slot].w : o4.w)].params;
+                wide = (const WideNode*)p->wide;
+                tris = (const float4*)p->tris;
+                wide_begin(k, o4.x, o4.y, o4.z, d4.x, d4.y, d4.z, tmax, SHADOW, p->wide_size);
+                loaded = true;
+                ++rays;
+            }
+            const uint32_t took = min((uint32_t)__popc(ended), avail);
+            pool_next += took;
+            if (took == 0 && exhausted && ended == 0xFFFFFFFFu) break;
+            continue;
+        }
+        const bool at_leaf = k.cur != kWideDone && (k.cur & kWideLeaf);
+        const uint32_t leaves = __ballot_sync(0xFFFFFFFFu, at_leaf);
+        const int live = __popc(~ended);
+        if (__popc(leaves) >= (live < PT_WIDE_BATCH ? live : PT_WIDE_BATCH)) {
+            if (at_leaf) {
+                wide_faces(k, tris, [&]() { return (const uint4*)p->nodes; }, dir);
+                if (k.done) k.cur = kWideDone; else wide_pop(k);
+            }
+        } else {
+#pragma unroll 1
+            for (int step = 0; step < PT_WIDE_STEPS && !(k.cur & kWideLeaf); ++step) {
+                if (wide_visit(k, wide)) wide_pop(k);
+                else { k.done = true; k.any = k.binary = false; k.cur = kWideDone; }  // guard failure
+            }
+        }
+    }
+    if (rays_traced) {
+        const uint32_t s = __reduce_add_sync(0xFFFFFFFFu, rays);
+        if (lane == 0 && s) atomicAdd(rays_traced, (unsigned long long)s);
+    }
+}
+
 __global__ void __launch_bounds__(128) wf_shade_kernel(const WfItem* __restrict__ items, WfState ws,
                                                        const uint32_t* __restrict__ queue, const uint32_t* count_ptr,
                                                        uint32_t* __restrict__ next_queue, uint32_t* next_count) {
@@ -273,6 +393,12 @@ struct ColdLane {
     __device__ __forceinline__ uint32_t u(uint32_t k) const { return c[k * 128]; }
     __device__ __forceinline__ void set(uint32_t k, float v) const { c[k * 128] = __float_as_uint(v); }
     __device__ __forceinline__ void set(uint32_t k, uint32_t v) const { c[k * 128] = v; }
+    __device__ __forceinline__ void set(uint32_t k, const void* v) const {  // words k, k + 1
+        set(k, (uint32_t)(uintptr_t)v);
+        set(k + 1, (uint32_t)((uintptr_t)v >> 32));
+    }
+    template <class T>
+    __device__ __forceinline__ const T* ptr(uint32_t k) const { return (const T*)((uintptr_t)u(k + 1) << 32 | u(k)); }
     __device__ __forceinline__ F3 f3at(uint32_t k) const { return f3(f(k), f(k + 1), f(k + 2)); }
     __device__ __forceinline__ void set3(uint32_t k, const F3& v) const { set(k, v.x); set(k + 1, v.y); set(k + 2, v.z); }
 };
@@ -500,6 +626,202 @@ __global__ void __launch_bounds__(128, PT_PATH_MIN_BLOCKS) wf_path_kernel(const 
     }
 }
 
+// Whole paths over four-wide records (every item has them).  A lane is in one of four groups, and the
+// warp runs one group's step at a time, so that each step's code runs for many lanes:
+//   * visit:  its ray's next record is tested;
+//   * faces:  its ray stands at a leaf, whose faces are tested;
+//   * shade:  its path's ray has hit a face: the integrator step, which leaves the next rays;
+//   * turn:   everything else that ends or starts a ray: misses and shadow results, finished paths
+//             (whose radiance is stored), camera rays of new paths, and the start of every walk.
+// Hits wait for each other apart from the turns: misses, shadow rays and finished paths are more, and
+// take a tenth of the shading code.  Each lane's own sequence of operations is that of path_fused.
+enum PathField : uint32_t {
+    kPo, kPoy, kPoz, kPd, kPdy, kPdz,              // the path's next (or current) ray
+    kPs, kPsg, kPsb, kPl, kPlg, kPlb,              // throughput, radiance
+    kPw, kPwy, kPwz, kPt, kPc, kPcg, kPcb,         // shadow ray: direction, far bound; contribution
+    kPbounces, kPslot, kPpixel, kPsample, kPitem, kPtris, kPtrisHi,
+    kPathFields
+};
+constexpr uint32_t kIdle = 0, kOnPath = 1, kOnShadow = 2, kToPath = 3, kToShadow = 4, kToEnd = 5;  // lane's ray, or its next
+constexpr uint32_t kRayMask = 7, kPathLambert = 8, kPathPending = 16;                             // and flags of its path
+
+template <int SH>
+__global__ void __launch_bounds__(128, PT_WIDE_PATH_BLOCKS) wf_wide_path_kernel(const WfItem* __restrict__ items,
+                                                      const WfSegment* __restrict__ segs, uint32_t nseg, uint32_t count,
+                                                      float* __restrict__ radiance, unsigned long long* fetch, uint32_t chunk,
+                                                      unsigned long long* rays_traced) {
+    const uint32_t lane = threadIdx.x & 31u;
+    __shared__ uint2 sstack[SH * 128];
+    __shared__ uint32_t sfield[kPathFields * 128];
+    const ColdLane cold{sfield + threadIdx.x};
+    WideWalkT<kWideStack, SH> k;
+    k.stack.base = sstack + threadIdx.x;
+    k.stack.stride = 128;
+    k.cur = kWideDone;
+    k.prim = kPrimNone;
+    uint32_t pool_next = 0, pool_end = 0, rays = 0, state = kIdle;
+    bool exhausted = false, ok = true;
+    const WideNode* wide = nullptr;
+    while (true) {
+        const bool ended = k.cur == kWideDone;
+        const bool hit = ended && (state & kRayMask) == kOnPath && k.prim != kPrimNone && ok;
+        const uint32_t turns = __ballot_sync(0xFFFFFFFFu, ended && !hit && !(state == kIdle && exhausted));
+        const uint32_t hits = __ballot_sync(0xFFFFFFFFu, hit);
+        const uint32_t leaves = __ballot_sync(0xFFFFFFFFu, !ended && (k.cur & kWideLeaf));
+        const uint32_t walks = __ballot_sync(0xFFFFFFFFu, !(k.cur & kWideLeaf));
+        const int nwalk = __popc(leaves | walks);
+        if (__popc(turns) >= PT_WIDE_TURNS || (turns && nwalk == 0 && __popc(hits) < PT_WIDE_SHADES)) {
+            uint32_t todo = state & kRayMask;
+            if (ended && !hit && todo != kIdle) {
+                if (todo == kOnPath || todo == kOnShadow) {
+                    ++rays;
+                    const WfItem& it = items[cold.u(kPitem)];
+                    const RenderParams* p = it.params;
+                    if (!ok) {
+                        raise_flag(p->err);
+                        todo = kToEnd;
+                    } else if (todo == kOnPath) {
+                        PathState s;
+                        s.src = cold.f3at(kPs);
+                        s.L = cold.f3at(kPl);
+                        shade_miss(*p, s);
+                        cold.set3(kPl, s.L);
+                        if (cold.u(kPbounces) == 0 && cold.u(kPsample) == 0 && it.primary) it.primary[cold.u(kPpixel)] = kPrimNone;
+                        todo = kToEnd;
+                    } else {
+                        if (k.prim == kPrimNone) cold.set3(kPl, vadd(cold.f3at(kPl), cold.f3at(kPc)));
+                        todo = (state & kPathPending) && !throughput_is_zero(cold.f3at(kPs)) ? kToPath : kToEnd;
+                    }
+                }
+                if (todo == kToEnd) {
+                    clamp_store(radiance + 3 * (size_t)cold.u(kPslot), cold.f3at(kPl));
+                    todo = kIdle;
+                }
+            }
+            // new paths for the idle lanes
+            const uint32_t need = __ballot_sync(0xFFFFFFFFu, ended && !hit && todo == kIdle);
+            if (need && !exhausted && pool_next >= pool_end) {
+                unsigned long long base = 0;
+                if (lane == 0) base = atomicAdd(fetch, (unsigned long long)chunk);
+                base = __shfl_sync(0xFFFFFFFFu, base, 0);
+                if (base >= count) {
+                    exhausted = true;
+                } else {
+                    pool_next = (uint32_t)base;
+                    pool_end = base + chunk < count ? (uint32_t)base + chunk : count;
+                }
+            }
+            const uint32_t avail = pool_end - pool_next;
+            const uint32_t rank = __popc(need & ((1u << lane) - 1u));
+            if (ended && !hit && todo == kIdle && rank < avail) {
+                const uint32_t slot = pool_next + rank;
+                const WfSegment sg = segs[find_segment(segs, nseg, slot)];
+                const RenderParams* p = items[sg.item].params;
+                wide = (const WideNode*)p->wide;
+                uint32_t pixel, sample;
+                F3 o, d;
+                path_camera(*p, sg.local_begin + (slot - sg.slot_base), pixel, sample, o, d);
+                cold.set3(kPo, o);
+                cold.set3(kPd, d);
+                cold.set3(kPs, f3(1.f, 1.f, 1.f));
+                cold.set3(kPl, f3(0.f, 0.f, 0.f));
+                cold.set(kPbounces, 0u);
+                cold.set(kPslot, slot);
+                cold.set(kPpixel, pixel);
+                cold.set(kPsample, sample);
+                cold.set(kPitem, sg.item);
+                cold.set(kPtris, p->tris);
+                state = kToPath;
+                todo = kToPath;
+            }
+            pool_next += min((uint32_t)__popc(need), avail);
+            if (ended && !hit) {
+                state = (state & ~kRayMask) | todo;
+                if (todo == kToPath || todo == kToShadow) {
+                    const bool shadow = todo == kToShadow;
+                    const F3 o = cold.f3at(kPo), d = cold.f3at(shadow ? kPw : kPd);
+                    const float tmax = shadow ? cold.f(kPt) : bitsf(0x7F800000u);
+                    const RenderParams* p = items[cold.u(kPitem)].params;
+                    wide_begin(k, o.x, o.y, o.z, d.x, d.y, d.z, tmax, shadow, p->wide_size);
+                    state = (state & ~kRayMask) | (shadow ? kOnShadow : kOnPath);
+                    ok = true;
+                } else {
+                    state = kIdle;
+                    k.binary = false;
+                }
+            }
+        } else if (hits && (nwalk == 0 || __popc(hits) >= PT_WIDE_SHADES)) {
+            if (hit) {
+                ++rays;
+                const WfItem& it = items[cold.u(kPitem)];
+                PathState s;
+                s.o = cold.f3at(kPo);
+                s.d = cold.f3at(kPd);
+                s.src = cold.f3at(kPs);
+                s.L = cold.f3at(kPl);
+                s.bounces = cold.u(kPbounces);
+                s.last_lambert = (state & kPathLambert) ? 1u : 0u;
+                const uint32_t pixel = cold.u(kPpixel), sample = cold.u(kPsample);
+                if (s.bounces == 0 && sample == 0 && it.primary) it.primary[pixel] = k.prim;
+                ShadowReq sh;
+                const bool more = shade_hit(*it.params, s, k.prim, k.leaf, k.u, k.v, k.w, pixel, sample, sh);
+                cold.set3(kPo, s.o);
+                cold.set3(kPd, s.d);
+                cold.set3(kPs, s.src);
+                cold.set3(kPl, s.L);
+                cold.set(kPbounces, s.bounces);
+                state = s.last_lambert ? kPathLambert : 0u;
+                if (sh.valid) {  // its origin is the next path ray's
+                    cold.set3(kPw, sh.wi);
+                    cold.set(kPt, sh.tmax);
+                    cold.set3(kPc, sh.contrib);
+                    state |= kToShadow | (more ? kPathPending : 0u);
+                } else {
+                    state |= more && !throughput_is_zero(s.src) ? kToPath : kToEnd;
+                }
+            }
+        } else if (leaves && __popc(leaves) >= (nwalk < PT_WIDE_BATCH_PATHS ? nwalk : PT_WIDE_BATCH_PATHS)) {
+            if (!ended && (k.cur & kWideLeaf)) {
+                auto dir = [&](float& x, float& y, float& z) {
+                    const F3 d = cold.f3at((state & kRayMask) == kOnShadow ? kPw : kPd);
+                    x = d.x; y = d.y; z = d.z;
+                };
+                wide_faces(k, cold.template ptr<float4>(kPtris),
+                           [&]() { return (const uint4*)items[cold.u(kPitem)].params->nodes; }, dir);
+                if (k.done) k.cur = kWideDone; else wide_pop(k);
+            }
+        } else if (walks) {
+#pragma unroll 1
+            for (int step = 0; step < PT_WIDE_PATH_STEPS && !(k.cur & kWideLeaf); ++step) {
+                if (wide_visit(k, wide)) {
+                    wide_pop(k);
+                } else {
+                    ok = false;
+                    k.cur = kWideDone;
+                }
+            }
+        } else {
+            break;  // every lane idle, no path left
+        }
+        // the rays that the records are not for, and those whose MinT rose
+        if (k.cur == kWideDone && k.binary) {
+            const bool shadow = (state & kRayMask) == kOnShadow;
+            const F3 o = cold.f3at(kPo), d = cold.f3at(shadow ? kPw : kPd);
+            const RenderParams* p = items[cold.u(kPitem)].params;
+            const BinaryRay ray{o.x, o.y, o.z, d.x, d.y, d.z, shadow ? cold.f(kPt) : bitsf(0x7F800000u), shadow};
+            BinaryHit b;
+            ok = wide_binary_walk((const uint4*)p->nodes, (const float4*)p->tris, p->num_nodes, &ray, &b);
+            k.prim = b.prim; k.leaf = b.leaf;
+            k.u = b.u; k.v = b.v; k.w = b.w;
+            k.binary = false;
+        }
+    }
+    if (rays_traced) {
+        const uint32_t sum = __reduce_add_sync(0xFFFFFFFFu, rays);
+        if (lane == 0 && sum) atomicAdd(rays_traced, (unsigned long long)sum);
+    }
+}
+
 __global__ void wf_advance_kernel(uint32_t* counters, uint32_t consumed) {
     counters[consumed] = 0;
     counters[2] = 0;
@@ -699,12 +1021,31 @@ cudaError_t launch_path_stage(const WfItem* items, const WfSegment* segs, uint32
     return cudaGetLastError();
 }
 
-cudaError_t path_stage(int cap, bool two_level, const WfItem* items, const WfSegment* segs, uint32_t nseg, uint32_t count,
+cudaError_t launch_wide_paths(const WfItem* items, const WfSegment* segs, uint32_t nseg, uint32_t count, float* radiance,
+                              unsigned long long* fetch, uint32_t chunk, unsigned long long* rays, cudaStream_t s) {
+    constexpr int SH = 16;
+    int dev = 0, sms = 0, per_sm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, wf_wide_path_kernel<SH>, 128, 0);
+    if (e != cudaSuccess) return e;
+    if (per_sm < 1) per_sm = 1;
+    uint64_t grid = (uint64_t)sms * per_sm;
+    const uint64_t grid_needed = (((uint64_t)count + chunk - 1) / chunk * 32 + 127) / 128;
+    if (grid > grid_needed) grid = grid_needed ? grid_needed : 1;
+    e = cudaMemsetAsync(fetch, 0, sizeof(unsigned long long), s);
+    if (e != cudaSuccess) return e;
+    wf_wide_path_kernel<SH><<<(unsigned)grid, 128, 0, s>>>(items, segs, nseg, count, radiance, fetch, chunk, rays);
+    return cudaGetLastError();
+}
+
+cudaError_t path_stage(const WfTuning& t, const WfItem* items, const WfSegment* segs, uint32_t nseg, uint32_t count,
                        float* radiance, unsigned long long* fetch, uint32_t chunk, unsigned long long* rays, cudaStream_t s) {
-    if (two_level) {  // the top level, the exit marker and the bottom level share the stack: the largest capacity
+    if (t.two_level) {  // the top level, the exit marker and the bottom level share the stack: the largest capacity
         return launch_path_stage<64, true>(items, segs, nseg, count, radiance, fetch, chunk, rays, s);
     }
-    switch (cap) {
+    if (t.wide) return launch_wide_paths(items, segs, nseg, count, radiance, fetch, chunk, rays, s);
+    switch (t.stack_cap) {
         case 24: return launch_path_stage<24, false>(items, segs, nseg, count, radiance, fetch, chunk, rays, s);
         case 32: return launch_path_stage<32, false>(items, segs, nseg, count, radiance, fetch, chunk, rays, s);
         case 48: return launch_path_stage<48, false>(items, segs, nseg, count, radiance, fetch, chunk, rays, s);
@@ -712,10 +1053,32 @@ cudaError_t path_stage(int cap, bool two_level, const WfItem* items, const WfSeg
     }
 }
 
+template <bool SHADOW, int THREADS>
+cudaError_t launch_wide_stage(const WfItem* items, const WfState& ws, const uint32_t* queue, const uint32_t* count_ptr,
+                              unsigned long long* fetch, const WfTuning& t, unsigned long long* rays, cudaStream_t s) {
+    int dev = 0, sms = 0, per_sm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, wf_wide_kernel<SHADOW, THREADS>, THREADS, 0);
+    if (e != cudaSuccess) return e;
+    if (per_sm < 1) per_sm = 1;
+    e = cudaMemsetAsync(fetch, 0, sizeof(unsigned long long), s);
+    if (e != cudaSuccess) return e;
+    wf_wide_kernel<SHADOW, THREADS><<<(unsigned)(sms * per_sm), THREADS, 0, s>>>(items, ws, queue, count_ptr, fetch, t.queue_chunk, rays);
+    return cudaGetLastError();
+}
+
 template <bool SHADOW>
-cudaError_t trace_stage(int cap, const WfItem* items, const WfState& ws, const uint32_t* queue, const uint32_t* count_ptr,
+cudaError_t trace_stage(const WfItem* items, const WfState& ws, const uint32_t* queue, const uint32_t* count_ptr,
                         unsigned long long* fetch, const WfTuning& t, unsigned long long* rays, cudaStream_t s) {
-    switch (cap) {
+    if (t.wide) {
+        switch (t.threads_per_block) {
+            case 64: return launch_wide_stage<SHADOW, 64>(items, ws, queue, count_ptr, fetch, t, rays, s);
+            case 128: return launch_wide_stage<SHADOW, 128>(items, ws, queue, count_ptr, fetch, t, rays, s);
+            default: return launch_wide_stage<SHADOW, 256>(items, ws, queue, count_ptr, fetch, t, rays, s);
+        }
+    }
+    switch (t.stack_cap) {
         case 24: return launch_trace_stage<24, SHADOW>(items, ws, queue, count_ptr, fetch, t, rays, s);
         case 32: return launch_trace_stage<32, SHADOW>(items, ws, queue, count_ptr, fetch, t, rays, s);
         case 48: return launch_trace_stage<48, SHADOW>(items, ws, queue, count_ptr, fetch, t, rays, s);
@@ -734,12 +1097,12 @@ cudaError_t bounce_stages(const WfItem* d_items, const WfSegment* d_segments, co
     uint32_t cur = 0;
     for (uint32_t b = 0; e == cudaSuccess && b < w.bounces; ++b) {
         const uint32_t nxt = cur ^ 1u;
-        e = trace_stage<false>(t.stack_cap, d_items, ws, ws.queue[cur], ws.counters + cur, fetch0, t, rays_traced, s);
+        e = trace_stage<false>(d_items, ws, ws.queue[cur], ws.counters + cur, fetch0, t, rays_traced, s);
         if (e != cudaSuccess) break;
         wf_shade_kernel<<<blocks, 128, 0, s>>>(d_items, ws, ws.queue[cur], ws.counters + cur, ws.queue[nxt], ws.counters + nxt);
         e = cudaGetLastError();
         if (e != cudaSuccess) break;
-        e = trace_stage<true>(t.stack_cap, d_items, ws, nullptr, ws.counters + 2, fetch1, t, rays_traced, s);
+        e = trace_stage<true>(d_items, ws, nullptr, ws.counters + 2, fetch1, t, rays_traced, s);
         if (e != cudaSuccess) break;
         wf_advance_kernel<<<1, 1, 0, s>>>(ws.counters, cur);
         e = cudaGetLastError();
@@ -757,7 +1120,7 @@ cudaError_t wf_launch_wave(const WfItem* d_items, const WfSegment* d_segments, c
     if (w.count == 0) return cudaSuccess;
     if (w.count > ws.capacity) return cudaErrorInvalidValue;
     if (!t.paths && !ws.ray_o) return cudaErrorInvalidValue;  // state carved for the path kernel only
-    cudaError_t e = t.paths ? path_stage(t.stack_cap, t.two_level, d_items, d_segments + w.seg_begin, w.seg_count, w.count,
+    cudaError_t e = t.paths ? path_stage(t, d_items, d_segments + w.seg_begin, w.seg_count, w.count,
                                          ws.radiance, (unsigned long long*)(ws.counters + 4), t.queue_chunk, rays_traced, s)
                             : bounce_stages(d_items, d_segments, w, ws, t, rays_traced, s);
     if (e != cudaSuccess) return e;

@@ -76,6 +76,7 @@ struct WfTuning {
     int stack_cap = 64;                // traversal stack entries
     bool paths = false;                // one thread per whole path instead of per-bounce kernels
     bool two_level = false;            // (paths only) some item is a two-level scene
+    bool wide = false;                 // every item has four-wide records
 };
 
 // One wave: `count` slots, `bounces` extend/shade/shadow iterations, and its ranges in the plan's

@@ -378,8 +378,8 @@ PT_HD bool wide_visit(WideWalkT<CAP, SH>& k, const WideNode* __restrict__ wide) 
 // Whether the binary walk would test the leaf of face (v0, v1, v2) at far bound min_t: the face's own
 // box lies in the leaf's, so where it passes the leaf's does; else the leaf's own decides.  `dir` gives
 // the ray's direction where its 1/d was cut.
-template <class K, class Dir>
-PT_HD bool wide_leaf_passes(const K& k, float4 q0, float4 q1, float4 q2, const uint4* __restrict__ nodes, float min_t, const Dir& dir) {
+template <class K, class Nodes, class Dir>
+PT_HD bool wide_leaf_passes(const K& k, float4 q0, float4 q1, float4 q2, const Nodes& nodes, float min_t, const Dir& dir) {
     RayState r;
     r.ox = k.r.ox; r.oy = k.r.oy; r.oz = k.r.oz;
     r.ix = k.r.ix; r.iy = k.r.iy; r.iz = k.r.iz;
@@ -394,18 +394,20 @@ PT_HD bool wide_leaf_passes(const K& k, float4 q0, float4 q1, float4 q2, const u
         if (box_hits_fast(r, lx, ly, lz, hx, hy, hz, min_t)) return true;
     }
     const uint32_t ni = fbits(q2.w);
-    const uint4 a = ldg(nodes + 2 * (size_t)ni), b = ldg(nodes + 2 * (size_t)ni + 1);
+    const uint4* q = nodes() + 2 * (size_t)ni;
+    const uint4 a = ldg(q), b = ldg(q + 1);
     return box_hits(r, bitsf(a.x), bitsf(a.y), bitsf(a.z), bitsf(a.w), bitsf(b.x), bitsf(b.y), min_t, false);
 }
 
 // The faces of leaf k.cur in leaf order, as the binary walk tests them; sets k.done when the walk ends
-// here (an any-hit ray accepted a face, or MinT rose and `binary` is set).
-template <int CAP, int SH, class Dir>
-PT_HD void wide_faces(WideWalkT<CAP, SH>& k, const float4* __restrict__ tris, const uint4* __restrict__ nodes, const Dir& dir) {
+// here (an any-hit ray accepted a face, or MinT rose and `binary` is set).  `nodes` gives the binary nodes,
+// which only large leaves and boxes to be tested exactly need.
+template <int CAP, int SH, class Nodes, class Dir>
+PT_HD void wide_faces(WideWalkT<CAP, SH>& k, const float4* __restrict__ tris, const Nodes& nodes, const Dir& dir) {
     uint32_t at = k.cur & kWideIndex, n = (k.cur >> 28) & 7u;
     if (n == kWideBig) {
         uint4 a, b;
-        ldg_node(nodes + 2 * (size_t)at, a, b);
+        ldg_node(nodes() + 2 * (size_t)at, a, b);
         at = b.z;
         n = b.w & 0xFFFFu;
     }

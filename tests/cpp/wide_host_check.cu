@@ -38,7 +38,7 @@ static bool walk(WideWalkT<CAP, SH>& k, const std::vector<WideNode>& wide, const
     while (k.cur != kWideDone) {
         ++steps;
         if (k.cur & kWideLeaf) {
-            wide_faces(k, tris.data(), nodes.data(), dir);
+            wide_faces(k, tris.data(), [&]() { return nodes.data(); }, dir);
             if (k.done) break;
         } else if (!wide_visit(k, wide.data())) {
             return false;

@@ -56,3 +56,49 @@ def test_large_leaf_and_grid_together(cuda_device):
     s = pb.Scene([copies(300, 0), grid(40)])
     same_hits(s, np.concatenate([axis_rays(50_000, 1), edge_case_rays(50_000, 2)]))
     s.close()
+
+
+AXIS_CAMERA = dict(eye=(0.0, 0.0, 7.0), look_at=(0.0, 0.0, 0.0), up=(0.0, 1.0, 0.0), fov=50.0)
+
+
+def loose(name):
+    """The scene over a tree of the caller's own whose boxes do not nest."""
+    meshes = scene(name)
+    nodes, pairs = pb.bvh_build(meshes)
+    nodes["bb"][np.nonzero(nodes["num_faces"] > 0)[0][::3], 3:6] += np.float32(0.25)
+    return pb.Scene(meshes, env=(51.0,) * 3, nodes=nodes, leaf_pairs=pairs)
+
+
+@pytest.mark.parametrize("size, spp", [((1, 1), 1), ((33, 33), 3), ((130, 67), 2), ((257, 255), 1)])
+@pytest.mark.parametrize("name", ["small", "boxes", "grid", "coincident"])
+def test_wide_frames_match_the_fused_walk(cuda_device, name, size, spp):
+    """The path and wavefront kernels over four-wide records against the one-thread-per-path kernel, with
+    a camera whose middle rays run along an axis."""
+    s = pb.Scene(scene(name), env=(51.0,) * 3)
+    args = (size[0], size[1], spp, 5, AXIS_CAMERA, 9)
+    for nee in (0, pb.RENDER_NEE):
+        film, prim = pb.render(s, *args, flags=nee | pb.RENDER_FUSED)
+        for pipe in (0, pb.RENDER_PERSISTENT, pb.RENDER_WAVEFRONT):
+            got, gprim = pb.render(s, *args, flags=nee | pipe)
+            assert got.tobytes() == film.tobytes() and gprim.tobytes() == prim.tobytes(), (name, pipe)
+    s.close()
+
+
+@pytest.mark.parametrize("pipeline", [pb.PIPELINE_WAVEFRONT, pb.PIPELINE_PATHS])
+@pytest.mark.parametrize("threads", [64, 128, 256])
+def test_batches_with_and_without_records(cuda_device, pipeline, threads):
+    scenes = [pb.Scene(scene("boxes"), env=(51.0,) * 3), loose("small"), pb.Scene(scene("small"), env=(51.0,) * 3)]
+    t = pb.default_tuning()
+    t.pipeline, t.threads_per_block = pipeline, threads
+    for pick in ([0, 2], [0, 1, 2]):
+        jobs = [(scenes[k], pb.render_desc(61 + 7 * k, 40, 3, 4, AXIS_CAMERA, k, pb.RENDER_NEE)) for k in pick]
+        b = pb.Batch(jobs, t)
+        b.run()
+        for i, (s, rd) in enumerate(jobs):
+            film, prim = pb.render(s, rd.width, rd.height, rd.spp, rd.max_depth, AXIS_CAMERA, int(rd.seed),
+                                   pb.RENDER_NEE | pb.RENDER_FUSED)
+            got, gprim = b.output(i)
+            assert got.tobytes() == film.tobytes() and gprim.tobytes() == prim.tobytes(), (pick, i)
+        b.close()
+    for s in scenes:
+        s.close()
