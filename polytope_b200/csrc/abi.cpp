@@ -54,41 +54,78 @@ int upload(void** dst, const T* src, size_t count, uint64_t& bytes) {
     return PT_OK;
 }
 
-// The four-wide records of the scene's tree, made on the device from the uploaded nodes.  A tree with
-// a box outside its parent's (only a caller's own tree can have one) or of extreme size gets none and
-// keeps the binary walk, as does one whose records do not fit in memory.
+float largest_coordinate(const pt_bvh_node& root) {
+    float m = 0.f;
+    for (int k = 0; k < 3; ++k) m = std::max(m, std::max(std::fabs(root.bb_min[k]), std::fabs(root.bb_max[k])));
+    return m;
+}
+
+// The four-wide records of the scene's trees (wide.cuh), made on the device from the uploaded nodes.  A
+// tree with a box outside its parent's (only a caller's own tree can have one) or of extreme size gets
+// none and keeps the binary walk, as does one whose records do not fit in memory.
 int make_wide(pt_scene* s, const HostScene& h) {
     if (h.wide_of.empty() || s->nan_boxes) return PT_OK;
-    const size_t n = h.wide_of.size();
-    for (int k = 0; k < 3; ++k)
-        s->wide_size = std::max(s->wide_size, std::max(std::fabs(h.nodes[0].bb_min[k]), std::fabs(h.nodes[0].bb_max[k])));
-    if (!(s->wide_size >= kWideSizeMin && s->wide_size <= kWideSizeMax)) return PT_OK;
-    // behind the records: the numbering and the flag, in the same allocation (scene creation waits for
-    // each cudaMalloc, now and then for milliseconds)
-    const size_t record_bytes = 64 * (size_t)h.num_wide;
-    if (cudaMalloc(&s->dev.wide, record_bytes + 4 * (n + 1)) != cudaSuccess) {
+    struct Tree { const void* nodes; const uint32_t* wide_of; uint32_t num_nodes, face_base; float size; bool faces; };
+    std::vector<Tree> trees;
+    std::vector<WideInstance> table(h.instances.size());
+    const size_t n = h.wide_of.size(), nt = h.top_wide_of.size();
+    // one allocation (scene creation waits for each cudaMalloc, now and then for milliseconds): the
+    // instance table, the records, then the numbering and the flag
+    const size_t table_bytes = (sizeof(WideInstance) * table.size() + 255) & ~(size_t)255, record_bytes = 64 * (size_t)h.num_wide;
+    char* base = nullptr;
+    if (cudaMalloc((void**)&base, table_bytes + record_bytes + 4 * (n + nt + 1)) != cudaSuccess) {
         cudaGetLastError();
-        s->dev.wide = nullptr;
         return PT_OK;
     }
-    uint32_t* tmp = (uint32_t*)((char*)s->dev.wide + record_bytes);
-    uint32_t outside = 0;
-    cudaError_t e = cudaMemcpy(tmp, h.wide_of.data(), 4 * n, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemset(tmp + n, 0, 4);
-    if (e == cudaSuccess) e = launch_wide_make(s->dev.nodes, tmp, (uint32_t)n, s->wide_size, 0, s->dev.wide, s->dev.tris, tmp + n, nullptr);
-    if (e == cudaSuccess) e = cudaMemcpy(&outside, tmp + n, 4, cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) return cuda_fail(e, "four-wide records");
-    if (outside) {
-        cudaFree(s->dev.wide);
-        s->dev.wide = nullptr;
+    s->wide_base = base;
+    char* records = base + table_bytes;
+    uint32_t* number = (uint32_t*)(records + record_bytes);
+    if (h.two_level) {
+        trees.push_back({s->dev.tlas_nodes, number + n, (uint32_t)nt, 0, largest_coordinate(h.tlas[0]), false});
+        for (const HostScene::Geometry& g : h.geometries)
+            trees.push_back({(const char*)s->dev.nodes + sizeof(pt_bvh_node) * (size_t)g.node_base, number + g.node_base, g.num_nodes,
+                             g.face_base, largest_coordinate(h.nodes[g.node_base]), true});
+        for (size_t i = 0; i < h.tlas.size(); ++i)
+            if (h.tlas[i].num_faces == 1) table[table.size() - 1 - h.tlas[i].offset].node = (uint32_t)i;
+        for (size_t i = 0; i < h.instances.size(); ++i) {
+            WideInstance& w = table[table.size() - 1 - i];  // instance 0 lies just before record 0
+            w.root = h.wide_of[h.instances[i].node_base];
+            w.size = largest_coordinate(h.nodes[h.instances[i].node_base]);
+        }
+    } else {
+        trees.push_back({s->dev.nodes, number, (uint32_t)n, 0, largest_coordinate(h.nodes[0]), true});
     }
+    bool fits = true;
+    for (const Tree& t : trees) fits = fits && t.size >= kWideSizeMin && t.size <= kWideSizeMax;
+    uint32_t outside = 0;
+    cudaError_t e = cudaSuccess;
+    if (fits) {
+        e = cudaMemcpy(number, h.wide_of.data(), 4 * n, cudaMemcpyHostToDevice);
+        if (e == cudaSuccess && nt) e = cudaMemcpy(number + n, h.top_wide_of.data(), 4 * nt, cudaMemcpyHostToDevice);
+        if (e == cudaSuccess && !table.empty())
+            e = cudaMemcpy(records - sizeof(WideInstance) * table.size(), table.data(), sizeof(WideInstance) * table.size(), cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = cudaMemset(number + n + nt, 0, 4);
+        for (const Tree& t : trees)
+            if (e == cudaSuccess)
+                e = launch_wide_make(t.nodes, t.wide_of, t.num_nodes, t.size, t.face_base, records, t.faces ? s->dev.tris : nullptr,
+                                     number + n + nt, nullptr);
+        if (e == cudaSuccess) e = cudaMemcpy(&outside, number + n + nt, 4, cudaMemcpyDeviceToHost);
+        if (e != cudaSuccess) return cuda_fail(e, "four-wide records");
+    }
+    if (!fits || outside) {
+        cudaFree(base);
+        s->wide_base = nullptr;
+        return PT_OK;
+    }
+    s->dev.wide = records;
+    s->wide_size = trees[0].size;
     return PT_OK;
 }
 
 void free_scene(pt_scene* s) {
     if (!s) return;
     DeviceGuard g(s->device);
-    void* bufs[] = {s->dev.nodes, s->dev.tris, s->dev.wide, s->dev.meshes, s->dev.prim_normals, s->dev.prim_tri,
+    void* bufs[] = {s->dev.nodes, s->dev.tris, s->wide_base, s->dev.meshes, s->dev.prim_normals, s->dev.prim_tri,
                     s->dev.light_tris, s->dev.light_cdf, s->dev.instances, s->dev.tlas_nodes, s->dev_in, s->dev_out,
                     s->err_flag, s->trace_err, s->ray_counters};
     for (void* b : bufs)
@@ -454,7 +491,6 @@ int create_from_host(const pt_scene_desc* desc, HostScene& h, pt_scene** out) {
         return false;
     };
     s->nan_boxes = has_nan(h.nodes) || has_nan(h.tlas);
-    if ((rc = make_wide(s.get(), h))) { free_scene(s.release()); return rc; }
     if (h.two_level) {
         s->two_level = true;
         s->dev.num_instances = (uint32_t)h.instances.size();
@@ -462,6 +498,7 @@ int create_from_host(const pt_scene_desc* desc, HostScene& h, pt_scene** out) {
         if ((rc = upload(&s->dev.instances, h.instances.data(), h.instances.size(), bytes))) { free_scene(s.release()); return rc; }
         if ((rc = upload(&s->dev.tlas_nodes, h.tlas.data(), h.tlas.size(), bytes))) { free_scene(s.release()); return rc; }
     }
+    if ((rc = make_wide(s.get(), h))) { free_scene(s.release()); return rc; }
     s->device_bytes = bytes;
     *out = s.release();
     return PT_OK;

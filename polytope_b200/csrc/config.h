@@ -81,3 +81,15 @@
 #ifndef PT_WIDE_PATH_STEPS
 #define PT_WIDE_PATH_STEPS 4
 #endif
+
+// Two-level scenes over four-wide records (queries and the persistent path kernel): resident blocks, and
+// lanes that must stand at an instance or an exit before those steps run.  Measured on a B200 (us, 1 M rays
+// on five instances of 82 k faces / ms, 1280x720x8 frame of five instances of 330 k faces through the
+// persistent kernel), over the binary trees before 633 / 14.5: 4 blocks 338 / 5.8, 3 blocks 390 / 7.6, 5
+// blocks 417 / 6.6, 6 blocks 473 / 7.5; entering from 4 or 16 lanes on within 2 %.
+#ifndef PT_WIDE_TL_BLOCKS
+#define PT_WIDE_TL_BLOCKS 4
+#endif
+#ifndef PT_WIDE_ENTERS
+#define PT_WIDE_ENTERS 8
+#endif

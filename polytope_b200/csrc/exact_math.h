@@ -11,8 +11,10 @@
 
 #ifdef __CUDACC__
 #define PT_HD __host__ __device__ __forceinline__
+#define PT_COLD inline __host__ __device__ __noinline__  // rare paths, kept out of line
 #else
 #define PT_HD inline
+#define PT_COLD inline
 #include <cmath>
 #endif
 

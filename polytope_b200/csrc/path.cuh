@@ -7,6 +7,7 @@
 
 #include "shade.cuh"
 #include "two_level.cuh"
+#include "wide.cuh"
 
 namespace pt {
 
@@ -92,40 +93,55 @@ PT_HD bool shade_miss(const RenderParams& p, PathState& s) {
     return false;
 }
 
-// The shading step of a flattened scene: the hit face's world vertices from the leaf-ordered
-// face records.
+// The hit face's world vertices and mesh: from the leaf-ordered face records of a flattened scene ...
+PT_HD void hit_vertices(const RenderParams& p, uint32_t leaf, F3& v0, F3& v1, F3& v2, uint32_t& mesh) {
+    load_face((const float4*)p.tris, leaf, v0, v1, v2, mesh);
+}
+
+// ... or of a two-level scene: the object-space face record carried to world space with its instance's
+// object_to_world, as the flattened scene's vertices were baked.
+PT_HD void hit_vertices_two_level(const RenderParams& p, uint32_t face, uint32_t inst, F3& v0, F3& v1, F3& v2, uint32_t& mesh) {
+    const float4* tris = (const float4*)p.tris;
+    const float4 q0 = ldg(tris + 3 * (size_t)face), q1 = ldg(tris + 3 * (size_t)face + 1), q2 = ldg(tris + 3 * (size_t)face + 2);
+    const DeviceInstance* in = (const DeviceInstance*)p.instances + inst;
+    float m[16];
+    for (int k = 0; k < 16; ++k) m[k] = ldg(in->o2w + k);
+    v0 = f3(q0.x, q0.y, q0.z);
+    v1 = f3(q0.w, q1.x, q1.y);
+    v2 = f3(q1.z, q1.w, q2.x);
+    apply_point_dev(m, v0.x, v0.y, v0.z);
+    apply_point_dev(m, v1.x, v1.y, v1.z);
+    apply_point_dev(m, v2.x, v2.y, v2.z);
+    mesh = ldg(&in->mesh);
+}
+
+// The shading step of either layout.
 PT_HD bool shade_hit(const RenderParams& p, PathState& s, uint32_t prim, uint32_t leaf, float u,
                                           float v, float w, uint32_t pixel, uint32_t sample, ShadowReq& sh) {
     sh.valid = false;
     if (prim == kPrimNone) return shade_miss(p, s);
     F3 v0, v1, v2;
     uint32_t mesh;
-    load_face((const float4*)p.tris, leaf, v0, v1, v2, mesh);
+    hit_vertices(p, leaf, v0, v1, v2, mesh);
     return shade_face(p, s, prim, v0, v1, v2, mesh, u, v, w, pixel, sample, sh);
 }
 
-// The shading step of a two-level scene: the object-space face record carried to world space
-// with its instance's object_to_world, as the flattened scene's vertices were baked.
 PT_HD bool shade_hit_two_level(const RenderParams& p, PathState& s, uint32_t prim, uint32_t face, uint32_t inst,
                                float u, float v, float w, uint32_t pixel, uint32_t sample, ShadowReq& sh) {
     sh.valid = false;
     if (prim == kPrimNone) return shade_miss(p, s);
-    const float4* tris = (const float4*)p.tris;
-    const float4 q0 = ldg(tris + 3 * (size_t)face), q1 = ldg(tris + 3 * (size_t)face + 1), q2 = ldg(tris + 3 * (size_t)face + 2);
-    const DeviceInstance* in = (const DeviceInstance*)p.instances + inst;
-    float m[16];
-    for (int k = 0; k < 16; ++k) m[k] = ldg(in->o2w + k);
-    F3 v0 = f3(q0.x, q0.y, q0.z), v1 = f3(q0.w, q1.x, q1.y), v2 = f3(q1.z, q1.w, q2.x);
-    apply_point_dev(m, v0.x, v0.y, v0.z);
-    apply_point_dev(m, v1.x, v1.y, v1.z);
-    apply_point_dev(m, v2.x, v2.y, v2.z);
-    return shade_face(p, s, prim, v0, v1, v2, ldg(&in->mesh), u, v, w, pixel, sample, sh);
+    F3 v0, v1, v2;
+    uint32_t mesh;
+    hit_vertices_two_level(p, face, inst, v0, v1, v2, mesh);
+    return shade_face(p, s, prim, v0, v1, v2, mesh, u, v, w, pixel, sample, sh);
 }
 
 PT_HD TwoLevelView two_level_view(const RenderParams& p) {
     return TwoLevelView{(const uint4*)p.nodes, (const float4*)p.tris, p.num_nodes, (const uint4*)p.top_nodes,
                         p.top_num_nodes, (const DeviceInstance*)p.instances, p.exact_tree != 0};
 }
+
+PT_COLD uint32_t path_sample(uint64_t path, uint32_t npix) { return (uint32_t)(path / npix); }
 
 // Camera ray of a path (pixel centre, or jittered with the (pixel, sample, 0xFFFF) RNG block).
 PT_HD void path_camera(const RenderParams& p, uint64_t path, uint32_t& pixel, uint32_t& sample,
@@ -135,8 +151,8 @@ PT_HD void path_camera(const RenderParams& p, uint64_t path, uint32_t& pixel, ui
         sample = (uint32_t)path / npix;
         pixel = (uint32_t)path - sample * npix;
     } else {
-        sample = (uint32_t)(path / npix);
-        pixel = (uint32_t)(path % npix);
+        sample = path_sample(path, npix);
+        pixel = (uint32_t)(path - (uint64_t)sample * npix);
     }
     const uint32_t x = pixel % p.width, y = pixel / p.width;
     float px = (float)x + 0.5f, py = (float)y + 0.5f;
@@ -157,34 +173,45 @@ PT_HD void clamp_store(float* out, const F3& L) {  // BoxFilter::AddSample clamp
 
 // ---- fused pipeline -------------------------------------------------------------------------
 
-// The fused path loop on a two-level scene (same steps as path_fused).
+// The fused path loop on a two-level scene: path_fused's steps, with one walk for path and shadow rays alike
+// (a lane whose path needs no shadow ray goes on to its next bounce beside the others' shadow rays, and the
+// walk's code is there once).
 template <int CAP>
 PT_HD uint32_t path_fused_two_level(const RenderParams& p, uint64_t path, float* out, uint32_t* primary) {
     const TwoLevelView view = two_level_view(p);
     const float inf = bitsf(0x7F800000u);
-    uint32_t pixel, sample;
+    uint32_t pixel, sample, rays = 0;
     PathState s;
     path_camera(p, path, pixel, sample, s.o, s.d);
     s.src = f3(1.f, 1.f, 1.f);
     s.L = f3(0.f, 0.f, 0.f);
     s.bounces = 0;
     s.last_lambert = 0;
-    uint32_t rays = 0;
-    while (!throughput_is_zero(s.src)) {
-        const TwoLevelHit h = traverse_two_level<false, CAP>(view, s.o.x, s.o.y, s.o.z, s.d.x, s.d.y, s.d.z, inf, false);
+    ShadowReq sh;
+    sh.valid = false;
+    bool more = true;
+    while (true) {
+        const bool shadow = sh.valid;  // a shadow ray starts where the next path ray does
+        const F3 d = shadow ? sh.wi : s.d;
+        const TwoLevelHit h = traverse_two_level<false, CAP>(view, s.o.x, s.o.y, s.o.z, d.x, d.y, d.z, shadow ? sh.tmax : inf, shadow);
         ++rays;
         if (h.r.overflow) { raise_flag(p.err); break; }
-        if (s.bounces == 0 && sample == 0 && primary) primary[pixel] = h.r.prim;
-        ShadowReq sh;
-        const bool more = shade_hit_two_level(p, s, h.r.prim, h.r.leaf, h.inst, h.r.u, h.r.v, h.r.w, pixel, sample, sh);
-        if (sh.valid) {
-            const TwoLevelHit t = traverse_two_level<false, CAP>(view, sh.o.x, sh.o.y, sh.o.z, sh.wi.x, sh.wi.y, sh.wi.z,
-                                                                 sh.tmax, true);
-            ++rays;
-            if (t.r.overflow) { raise_flag(p.err); break; }
-            if (t.r.prim == kPrimNone) s.L = vadd(s.L, sh.contrib);
+        if (shadow) {
+            if (h.r.prim == kPrimNone) s.L = vadd(s.L, sh.contrib);
+            sh.valid = false;
+        } else {
+            if (s.bounces == 0 && sample == 0 && primary) primary[pixel] = h.r.prim;
+            if (h.r.prim == kPrimNone) {
+                shade_miss(p, s);
+                break;
+            }
+            F3 v0, v1, v2;
+            uint32_t mesh;
+            hit_vertices_two_level(p, h.r.leaf, h.inst, v0, v1, v2, mesh);
+            more = shade_face(p, s, h.r.prim, v0, v1, v2, mesh, h.r.u, h.r.v, h.r.w, pixel, sample, sh);
+            if (sh.valid) continue;
         }
-        if (!more) break;
+        if (!more || throughput_is_zero(s.src)) break;
     }
     clamp_store(out, s.L);
     return rays;
@@ -224,6 +251,78 @@ PT_HD uint32_t path_fused(const RenderParams& p, uint64_t path, float* out, uint
             if (t.prim == kPrimNone) s.L = vadd(s.L, sh.contrib);
         }
         if (!more) break;
+    }
+    clamp_store(out, s.L);
+    return rays;
+}
+
+// ---- fused pipeline over four-wide records ------------------------------------------------------
+
+// One ray's whole walk (k set up by wide_begin for direction d).  False on a guard failure.
+template <class K>
+PT_HD bool wide_trace(K& k, const RenderParams& p, const F3& d, float tmax) {
+    auto dir = [&](float& x, float& y, float& z) { x = d.x; y = d.y; z = d.z; };
+    while (k.cur != kWideDone) {
+        while (!(k.cur & kWideLeaf)) {
+            if (!wide_visit(k, (const WideNode*)p.wide)) return false;
+            wide_pop(k);
+        }
+        if (k.cur == kWideDone) break;
+        wide_faces(k, (const float4*)p.tris, [&]() { return (const uint4*)p.nodes; }, dir, []() { return 0u; });
+        if (k.done) break;
+        wide_pop(k);
+    }
+    if (!k.binary) return true;
+    const BinaryRay ray{k.r.ox, k.r.oy, k.r.oz, d.x, d.y, d.z, tmax, k.any};
+    BinaryHit b;
+    const bool ok = wide_binary_walk((const uint4*)p.nodes, (const float4*)p.tris, p.num_nodes, &ray, &b);
+    k.prim = b.prim; k.leaf = b.leaf;
+    k.u = b.u; k.v = b.v; k.w = b.w;
+    return ok;
+}
+
+// path_fused with one walk for path and shadow rays, as path_fused_two_level.  stack: this lane's entries in
+// shared memory, `stride` apart.
+template <int SH>
+PT_HD uint32_t path_wide(const RenderParams& p, uint64_t path, float* out, uint32_t* primary, uint2* stack, uint32_t stride) {
+    const float inf = bitsf(0x7F800000u);
+    uint32_t pixel, sample, rays = 0;
+    PathState s;
+    path_camera(p, path, pixel, sample, s.o, s.d);
+    s.src = f3(1.f, 1.f, 1.f);
+    s.L = f3(0.f, 0.f, 0.f);
+    s.bounces = 0;
+    s.last_lambert = 0;
+    WideWalkT<kWideStack, SH> k;
+    k.stack.base = stack;
+    k.stack.stride = stride;
+    ShadowReq sh;
+    sh.valid = false;
+    bool more = true;
+    while (true) {
+        const bool shadow = sh.valid;  // a shadow ray starts where the next path ray does
+        const F3 d = shadow ? sh.wi : s.d;
+        const float tmax = shadow ? sh.tmax : inf;
+        wide_begin(k, s.o.x, s.o.y, s.o.z, d.x, d.y, d.z, tmax, shadow, p.wide_size);
+        const bool ok = wide_trace(k, p, d, tmax);
+        ++rays;
+        if (!ok) { raise_flag(p.err); break; }
+        if (shadow) {
+            if (k.prim == kPrimNone) s.L = vadd(s.L, sh.contrib);
+            sh.valid = false;
+        } else {
+            if (s.bounces == 0 && sample == 0 && primary) primary[pixel] = k.prim;
+            if (k.prim == kPrimNone) {
+                shade_miss(p, s);
+                break;
+            }
+            F3 v0, v1, v2;
+            uint32_t mesh;
+            hit_vertices(p, k.leaf, v0, v1, v2, mesh);
+            more = shade_face(p, s, k.prim, v0, v1, v2, mesh, k.u, k.v, k.w, pixel, sample, sh);
+            if (sh.valid) continue;
+        }
+        if (!more || throughput_is_zero(s.src)) break;
     }
     clamp_store(out, s.L);
     return rays;

@@ -95,6 +95,9 @@ struct HostScene {  // host copy of everything a scene handle uploads
     std::vector<uint32_t> prim_base;
     std::vector<uint32_t> wide_of;    // four-wide record that starts at each node (empty: none are made)
     uint32_t num_wide = 0;
+    std::vector<uint32_t> top_wide_of;  // two-level: the same for the top level, whose records come first
+    struct Geometry { uint32_t node_base, num_nodes, face_base; };
+    std::vector<Geometry> geometries;
     // two-level layout (pt_scene_create_two_level): `nodes` / `tris` then hold every distinct
     // geometry's object-space tree and faces back to back, and these the instances and the top
     // level over their world boxes
@@ -111,11 +114,19 @@ int prepare_two_level_host(const pt_scene_desc* desc, HostScene& out);
 // both layouts.
 void prepare_shading_host(const pt_scene_desc* desc, const WorldMeshes& w, HostScene& h);
 
+// Two-level scenes: an instance's four-wide tree.  Instance i is entry -1 - i before record 0.
+struct WideInstance {
+    uint32_t root;   // first record of the instance's tree
+    float size;      // largest coordinate of that tree's boxes
+    uint32_t node;   // top-level leaf that holds the instance
+    uint32_t pad;
+};
+
 struct SceneDev {
     // traversal data
     void* nodes = nullptr;        // num_nodes * 32 B  (pt_bvh_node)
     void* tris = nullptr;         // num_prims * 48 B  (3 x float4 per leaf-ordered entry)
-    void* wide = nullptr;         // four-wide records of the tree (wide.cuh), 64 B each, or null
+    void* wide = nullptr;         // four-wide records of the trees (wide.cuh), 64 B each, or null
     // shading data
     void* meshes = nullptr;       // num_meshes * DeviceMesh
     void* prim_normals = nullptr; // num_prims * 9 floats (world vertex normals by prim id) or null
@@ -160,7 +171,8 @@ struct pt_scene {
     void* err_flag = nullptr;
     void* trace_err = nullptr;
     bool two_level = false;  // made by pt_scene_create_two_level
-    float wide_size = 0.f;   // largest coordinate of the tree's boxes (wide.cuh)
+    void* wide_base = nullptr;  // allocation that holds dev.wide
+    float wide_size = 0.f;      // largest coordinate of the (top-level) tree's boxes
     bool nan_boxes = false;  // some tree box holds a NaN (every ray then takes the exact box test)
     // ray counters of the persistent trace kernel: one per launch in flight, taken round-robin
     void* ray_counters = nullptr;

@@ -31,15 +31,39 @@ static_assert(sizeof(pt::MeshRec) == sizeof(pt::DeviceMesh) && alignof(pt::MeshR
 
 namespace pt {
 
-// 8 resident blocks of 128 per SM (64 registers, some spilled) instead of the 96 registers the
-// compiler picks unbounded: on a B200 the 6.55 M-face frame 1362 -> 1691 Msamples/s (flattened)
-// and 1073 -> 1256 (two-level); 6, 7, 9, 10 and 12 blocks measured 1491, 1600, 1576, 1532, 1532.
+// The walk over the binary trees: two-level scenes, and flattened ones without four-wide records.  8
+// resident blocks of 128 per SM (64 registers, some spilled): on a B200 the 1280x720x8 frame of five
+// instances of 330 k faces takes 4.27 ms two-level; 4, 5, 6, 7 and 10 blocks measured 5.63, 4.95, 4.68,
+// 4.38, 4.49 (with a walk each for path and shadow rays, twice the code, 4.45 at 8 blocks).
+#ifndef PT_FUSED_BLOCKS
+#define PT_FUSED_BLOCKS 8
+#endif
 template <bool TWO_LEVEL>
-__global__ void __launch_bounds__(128, 8) path_kernel(const RenderParams p, uint64_t first, uint32_t count,
+__global__ void __launch_bounds__(128, PT_FUSED_BLOCKS) path_kernel(const RenderParams p, uint64_t first, uint32_t count,
                                                    float* __restrict__ radiance, uint32_t* __restrict__ primary) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t rays = 0;
-    if (i < count) rays = path_fused<kStackCap, TWO_LEVEL>(p, first + i, radiance + 3 * (size_t)i, primary);
+    if (i < count) rays = TWO_LEVEL ? path_fused_two_level<kStackCap>(p, first + i, radiance + 3 * (size_t)i, primary)
+                                   : path_fused(p, first + i, radiance + 3 * (size_t)i, primary);
+    if (p.rays_traced) {
+        const uint32_t sum = __reduce_add_sync(0xFFFFFFFFu, rays);
+        if ((threadIdx.x & 31u) == 0 && sum) atomicAdd(p.rays_traced, (unsigned long long)sum);
+    }
+}
+
+// Flattened scenes over their four-wide records, with the first 16 stack entries of a lane in shared memory.
+// On a B200 the 1920x1080x16 frame of 3.9 M faces takes 9.8 ms against 11.0 over the binary tree; 4, 5, 6,
+// 7 and 10 blocks measured 11.5, 10.4, 10.3, 10.2, 10.7.
+#ifndef PT_WIDE_FUSED_BLOCKS
+#define PT_WIDE_FUSED_BLOCKS 8
+#endif
+__global__ void __launch_bounds__(128, PT_WIDE_FUSED_BLOCKS) path_wide_kernel(const RenderParams p, uint64_t first, uint32_t count,
+                                                                            float* __restrict__ radiance,
+                                                                            uint32_t* __restrict__ primary) {
+    __shared__ uint2 sstack[16 * 128];
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t rays = 0;
+    if (i < count) rays = path_wide<16>(p, first + i, radiance + 3 * (size_t)i, primary, sstack + threadIdx.x, 128);
     if (p.rays_traced) {
         const uint32_t sum = __reduce_add_sync(0xFFFFFFFFu, rays);
         if ((threadIdx.x & 31u) == 0 && sum) atomicAdd(p.rays_traced, (unsigned long long)sum);
@@ -107,7 +131,9 @@ cudaError_t upload_async(void* dst, const void* src, size_t bytes, cudaStream_t 
 cudaError_t launch_path_wave(const RenderParams& p, uint64_t first, uint32_t count, float* radiance, uint32_t* primary,
                              cudaStream_t s) {
     if (!count) return cudaSuccess;
-    if (p.instances)
+    if (p.wide && !p.instances)
+        path_wide_kernel<<<(count + 127) / 128, 128, 0, s>>>(p, first, count, radiance, primary);
+    else if (p.instances)
         path_kernel<true><<<(count + 127) / 128, 128, 0, s>>>(p, first, count, radiance, primary);
     else
         path_kernel<false><<<(count + 127) / 128, 128, 0, s>>>(p, first, count, radiance, primary);
@@ -255,9 +281,9 @@ int enqueue_frame(pt_scene* s, const pt_render_desc* desc, float* rgb_d, uint32_
     p.err = err;
     // Pipelines: the persistent path kernel unless PT_RENDER_FUSED or PT_RENDER_WAVEFRONT is given
     // (the wave engine runs both the queue-based kernels and the persistent path kernel).
-    // two-level scenes default to the fused kernel: their persistent walk measured slower (599
-    // against 819 Msamples/s on the 6.5 M-face instanced frame), the top-level steps and instance
-    // entries interrupting the warp-voted node steps; PT_RENDER_PERSISTENT still selects it
+    // two-level scenes default to the fused kernel: coherent paths cross their instances together there,
+    // while the persistent kernel's crossings interrupt its steps (1280x720x8 frame of five instances:
+    // 4.4 ms fused, 5.9 persistent, 8.0 over the binary trees)
     const bool fused = (desc->flags & PT_RENDER_FUSED) != 0 || (s->two_level && !(desc->flags & PT_RENDER_PERSISTENT));
     const bool persistent = !fused && (desc->flags & PT_RENDER_WAVEFRONT) == 0;
     const bool wavefront = !fused;

@@ -166,9 +166,14 @@ int prepare_two_level_host(const pt_scene_desc* desc, HostScene& h) {
         BuiltTree t;
         rc = build_bvh(&obj, 1, wo, 0, t);
         if (rc) return rc;
-        uint32_t depth = 0;
-        rc = validate_tree(t.nodes.data(), (uint32_t)t.nodes.size(), wo.num_prims, &depth);
+        uint32_t depth = 0, records = 0;
+        std::vector<uint32_t> wide_of;
+        rc = validate_tree(t.nodes.data(), (uint32_t)t.nodes.size(), wo.num_prims, &depth, &wide_of, &records);
         if (rc) return rc;
+        h.geometries.push_back({(uint32_t)h.nodes.size(), (uint32_t)t.nodes.size(), (uint32_t)(h.tris.size() / 12)});
+        for (uint32_t& r : wide_of) r = r == kNotWide ? r : r + h.num_wide;
+        h.wide_of.insert(h.wide_of.end(), wide_of.begin(), wide_of.end());
+        h.num_wide += records;
         h.max_depth = std::max(h.max_depth, depth);
         // bottom-level node indices share the walk stack with tagged entries (bits 30 and 31)
         if ((uint64_t)h.nodes.size() + t.nodes.size() >= (1ull << 30) || (uint64_t)h.tris.size() / 12 + wo.num_prims > 0xFFFFFFF0ull)
@@ -226,9 +231,16 @@ int prepare_two_level_host(const pt_scene_desc* desc, HostScene& h) {
     h.tlas_depth = top.depth;
     h.instances.resize(desc->num_meshes);
     for (size_t i = 0; i < top.order.size(); ++i) h.instances[i] = inst[top.order[i]];
-    uint32_t tdepth = 0;
-    rc = validate_tree(h.tlas.data(), (uint32_t)h.tlas.size(), (uint32_t)h.instances.size(), &tdepth);
+    uint32_t tdepth = 0, records = 0;
+    rc = validate_tree(h.tlas.data(), (uint32_t)h.tlas.size(), (uint32_t)h.instances.size(), &tdepth, &h.top_wide_of, &records);
     if (rc) return fail(rc, std::string("top-level tree: ") + pt_last_error());
+    if (h.wide_of.size() == h.nodes.size() && !h.top_wide_of.empty() && h.nodes.size() < (1u << 28)) {
+        for (uint32_t& r : h.wide_of) r = r == kNotWide ? r : r + records;  // the top level's records come first
+        h.num_wide += records;
+    } else {
+        h.wide_of.clear();
+        h.num_wide = 0;
+    }
     h.two_level = true;
     h.num_prims = w.num_prims;
     h.prim_base = w.prim_base;

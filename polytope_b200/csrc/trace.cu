@@ -10,6 +10,7 @@
 #include "launch.h"
 #include "traverse.cuh"
 #include "two_level.cuh"
+#include "shade.cuh"
 #include "wide.cuh"
 
 namespace pt {
@@ -172,10 +173,10 @@ __global__ void __launch_bounds__(128) wide_make_kernel(const uint4* __restrict_
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= num_nodes) return;
     bool ok = true;
-    if ((nodes[2 * (size_t)i + 1].w & 0xFFFFu) != 0) ok = wide_mark_leaf(nodes, i, face_base, tris);
+    if (tris && (nodes[2 * (size_t)i + 1].w & 0xFFFFu) != 0) ok = wide_mark_leaf(nodes, i, face_base, tris);
     if (wide_of[i] != 0xFFFFFFFFu) {
         WideNode w;
-        ok = wide_make(nodes, wide_of, i, size, w) && ok;
+        ok = wide_make(nodes, wide_of, i, size, face_base, w) && ok;
         const uint4* src = (const uint4*)&w;
         uint4* dst = (uint4*)(wide + wide_of[i]);
 #pragma unroll
@@ -197,10 +198,13 @@ cudaError_t launch_wide_make(const void* nodes, const uint32_t* wide_of, uint32_
 // still walk), then those test their faces together; lanes whose ray has ended wait until PT_WIDE_REFILL
 // of them store their hits and take new rays together.  A batch smaller than the resident warps spreads
 // over all of them, a few rays a warp, and needs neither counter nor memset.
-template <int SH>
-__global__ void __launch_bounds__(128, PT_WIDE_BLOCKS) trace_wide_kernel(const WideNode* __restrict__ wide, const uint4* __restrict__ nodes,
+// TL: a two-level scene (v): lanes at a top-level leaf or an exit marker enter or leave their instance
+// PT_WIDE_ENTERS at a time.
+template <int SH, bool TL>
+__global__ void __launch_bounds__(128, TL ? PT_WIDE_TL_BLOCKS : PT_WIDE_BLOCKS) trace_wide_kernel(const WideNode* __restrict__ wide, const uint4* __restrict__ nodes,
                                                             const float4* __restrict__ tris, uint32_t num_nodes,
-                                                            const float4* __restrict__ rays, uint4* __restrict__ hits, uint32_t n,
+                                                            const uint4* __restrict__ top, uint32_t num_top,
+                                                            const DeviceInstance* __restrict__ inst, const float4* __restrict__ rays, uint4* __restrict__ hits, uint32_t n,
                                                             int* err, unsigned long long* counter, uint32_t chunk, float size) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t warp = blockIdx.x * 4 + (threadIdx.x >> 5);
@@ -209,14 +213,24 @@ __global__ void __launch_bounds__(128, PT_WIDE_BLOCKS) trace_wide_kernel(const W
     bool exhausted = false, loaded = false;  // loaded: the lane holds a ray whose hit is not yet stored
     uint32_t idx = 0;
     __shared__ uint2 sstack[SH > 0 ? SH * 128 : 1];
+    __shared__ uint32_t sinst[TL ? 128 : 1];  // the instance that the lane's walk is in, and MinT at its entry
+    __shared__ float sentry[TL ? 128 : 1];
+    bool sure = true;                         // a face was accepted in it: its box has passed
+    bool inside = !TL;                        // the walk is in an instance (or the scene is flattened)
     WideWalkT<kWideStack, SH> k;
     k.stack.base = sstack + threadIdx.x;
     k.stack.stride = 128;
     k.cur = kWideDone;
     k.binary = false;
+    // the direction of the ray that k.r was set up for
     auto dir = [&](float& x, float& y, float& z) {
-        const float4 d = rays[2 * (size_t)idx + 1];
-        x = d.x; y = d.y; z = d.z;
+        const float4 r1 = rays[2 * (size_t)idx + 1];
+        x = r1.x; y = r1.y; z = r1.z;
+        if constexpr (TL) {
+            F3 o = f3(0.f, 0.f, 0.f), d = f3(r1.x, r1.y, r1.z);
+            wide_to_object(inst + sinst[threadIdx.x], o, d);
+            x = d.x; y = d.y; z = d.z;
+        }
     };
     while (true) {
         // lanes whose ray has ended store its hit and take the next ray, PT_WIDE_REFILL at a time
@@ -229,7 +243,13 @@ __global__ void __launch_bounds__(128, PT_WIDE_BLOCKS) trace_wide_kernel(const W
                     const float4 r0 = rays[2 * (size_t)idx], r1 = rays[2 * (size_t)idx + 1];
                     const BinaryRay ray{r0.x, r0.y, r0.z, r1.x, r1.y, r1.z, r0.w, k.any};
                     BinaryHit b;
-                    ok = wide_binary_walk(nodes, tris, num_nodes, &ray, &b);
+                    if constexpr (TL) {
+                        const TwoLevelView view{nodes, tris, num_nodes, top, num_top, inst, false};
+                        uint32_t hit_inst;
+                        ok = wide_two_level_walk(&view, &ray, &b, &hit_inst);
+                    } else {
+                        ok = wide_binary_walk(nodes, tris, num_nodes, &ray, &b);
+                    }
                     h = make_uint4(b.prim, __float_as_uint(b.t), __float_as_uint(b.u), __float_as_uint(b.v));
                 } else {
                     h = make_uint4(k.prim, __float_as_uint(k.min_t), __float_as_uint(k.u), __float_as_uint(k.v));
@@ -261,6 +281,7 @@ __global__ void __launch_bounds__(128, PT_WIDE_BLOCKS) trace_wide_kernel(const W
                 const float4 r0 = ld_stream(rays + 2 * (size_t)idx);
                 const float4 r1 = ld_stream(rays + 2 * (size_t)idx + 1);
                 wide_begin(k, r0.x, r0.y, r0.z, r1.x, r1.y, r1.z, r0.w, (__float_as_uint(r1.w) & 1u) != 0, size);
+                inside = !TL;
                 loaded = true;
             }
             const uint32_t took = min((uint32_t)__popc(ended), avail);
@@ -268,12 +289,63 @@ __global__ void __launch_bounds__(128, PT_WIDE_BLOCKS) trace_wide_kernel(const W
             if (took == 0 && exhausted && ended == 0xFFFFFFFFu) break;
             continue;
         }
-        const bool at_leaf = k.cur != kWideDone && (k.cur & kWideLeaf);
+        const bool crosses = TL && k.cur != kWideDone && (k.cur == kWideExit || ((k.cur & kWideLeaf) && !inside));
+        const bool at_leaf = k.cur != kWideDone && (k.cur & kWideLeaf) && !crosses;
         const uint32_t leaves = __ballot_sync(0xFFFFFFFFu, at_leaf);
-        const uint32_t live = __popc(~ended);
+        uint32_t live = __popc(~ended);
+        if constexpr (TL) {
+            const uint32_t crossing = __ballot_sync(0xFFFFFFFFu, crosses);
+            live -= __popc(crossing);  // the lanes that walk
+            if (__popc(crossing) >= PT_WIDE_ENTERS || (crossing && live == 0)) {
+                if (crosses) {
+                    const float4 r0 = rays[2 * (size_t)idx], r1 = rays[2 * (size_t)idx + 1];
+                    F3 o = f3(r0.x, r0.y, r0.z), d = f3(r1.x, r1.y, r1.z);
+                    if (k.cur == kWideExit) {
+                        inside = false;
+                        wide_pop(k);
+                    }
+                    const bool enters = (k.cur & kWideLeaf) && k.cur != kWideDone;
+                    if (k.cur != kWideDone) {  // into an instance, or back to a top-level record
+                        const uint32_t ii = k.cur & kWideIndex;
+                        uint4 wi = make_uint4(0u, __float_as_uint(size), 0u, 0u);
+                        if (enters) {
+                            sinst[threadIdx.x] = ii;
+                            sentry[threadIdx.x] = k.min_t;
+                            sure = false;
+                            wide_to_object(inst + ii, o, d);
+                            wi = wide_instance(wide, ii);
+                        }
+                        ray_setup(k.r, o.x, o.y, o.z, d.x, d.y, d.z);
+                        const bool fits = wide_cut(k.r, k.cut, __uint_as_float(wi.y));
+                        if (enters) {
+                            inside = wide_enter(k, wi.x, fits);
+                            if (!inside) {
+                                k.any = k.any && k.binary;  // a guard failure is no any-hit result
+                                k.cur = kWideDone;
+                            }
+                        }
+                    }
+                }
+                continue;
+            }
+        }
         if (__popc(leaves) >= (live < PT_WIDE_BATCH ? live : PT_WIDE_BATCH)) {
             if (at_leaf) {
-                wide_faces(k, tris, [&]() { return nodes; }, dir);
+                if constexpr (TL) {
+                    const DeviceInstance* in = inst + sinst[threadIdx.x];
+                    if (wide_faces(k, tris, [&]() { return nodes + 2 * (size_t)ldg(&in->node_base); }, dir,
+                                   [&]() { return ldg(&in->face_base); })) {
+                        k.prim += ldg(&in->prim_base);
+                        if (!sure) {
+                            const float4 r0 = rays[2 * (size_t)idx], r1 = rays[2 * (size_t)idx + 1];
+                            if (!wide_instance_passes(wide, top, sinst[threadIdx.x], r0.x, r0.y, r0.z, r1.x, r1.y, r1.z, sentry[threadIdx.x]))
+                                k.binary = k.done = true;
+                            sure = true;
+                        }
+                    }
+                } else {
+                    wide_faces(k, tris, [&]() { return nodes; }, dir, []() { return 0u; });
+                }
                 if (k.done) k.cur = kWideDone; else wide_pop(k);
             }
         } else {
@@ -315,6 +387,31 @@ __global__ void __launch_bounds__(128) trace_two_level_kernel(const TwoLevelView
 
 cudaError_t launch_trace(const TraceArgs& a, cudaStream_t s) {
     if (a.n == 0) return cudaSuccess;
+    if (a.wide && a.counter && !a.node_tests && !a.tri_tests && a.n < 0xFFFF0000ull) {  // 32-bit ray numbers
+        const int sh = a.shared_stack;
+        auto pick = [sh](auto k0, auto k8, auto k16, auto k24, auto k32) {
+            return sh >= 32 ? k32 : sh >= 24 ? k24 : sh >= 16 ? k16 : sh >= 8 ? k8 : k0;
+        };
+        auto kern = a.instances ? pick(trace_wide_kernel<0, true>, trace_wide_kernel<8, true>, trace_wide_kernel<16, true>,
+                                       trace_wide_kernel<24, true>, trace_wide_kernel<32, true>)
+                                : pick(trace_wide_kernel<0, false>, trace_wide_kernel<8, false>, trace_wide_kernel<16, false>,
+                                       trace_wide_kernel<24, false>, trace_wide_kernel<32, false>);
+        int dev = 0, sms = 0, per_sm = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 128, 0);
+        if (e != cudaSuccess) return e;
+        const uint64_t warps = (uint64_t)sms * (per_sm < 1 ? 1 : per_sm) * 4;
+        uint64_t ch = a.chunk ? a.chunk : 64u;
+        ch = std::max<uint64_t>(1, std::min(ch, (a.n + warps - 1) / warps));
+        const uint64_t grid = std::min<uint64_t>(warps / 4, ((a.n + ch - 1) / ch + 3) / 4);
+        if (grid * 4 * ch < a.n) e = cudaMemsetAsync(a.counter, 0, sizeof(unsigned long long), s);
+        if (e != cudaSuccess) return e;
+        kern<<<(unsigned)grid, 128, 0, s>>>((const WideNode*)a.wide, (const uint4*)a.nodes, (const float4*)a.tris, a.num_nodes,
+                                            (const uint4*)a.top_nodes, a.top_num_nodes, (const DeviceInstance*)a.instances, (const float4*)a.rays, (uint4*)a.hits, (uint32_t)a.n, a.err,
+                                            (unsigned long long*)a.counter, (uint32_t)ch, a.wide_size);
+        return cudaGetLastError();
+    }
     if (a.instances) {
         const TwoLevelView v{(const uint4*)a.nodes, (const float4*)a.tris, a.num_nodes, (const uint4*)a.top_nodes,
                              a.top_num_nodes, (const DeviceInstance*)a.instances, a.exact_tree};
@@ -334,22 +431,6 @@ cudaError_t launch_trace(const TraceArgs& a, cudaStream_t s) {
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         const bool counted = a.node_tests || a.tri_tests;
         const int sh = a.shared_stack;
-        if (a.wide && !counted && a.n < 0xFFFF0000ull) {  // 32-bit ray numbers
-            auto kern = sh >= 32 ? trace_wide_kernel<32> : sh >= 24 ? trace_wide_kernel<24> : sh >= 16 ? trace_wide_kernel<16>
-                        : sh >= 8 ? trace_wide_kernel<8> : trace_wide_kernel<0>;
-            cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 128, 0);
-            if (e != cudaSuccess) return e;
-            const uint64_t warps = (uint64_t)sms * (per_sm < 1 ? 1 : per_sm) * 4;
-            uint64_t ch = a.chunk ? a.chunk : 64u;
-            ch = std::max<uint64_t>(1, std::min(ch, (a.n + warps - 1) / warps));
-            const uint64_t grid = std::min<uint64_t>(warps / 4, ((a.n + ch - 1) / ch + 3) / 4);
-            if (grid * 4 * ch < a.n) e = cudaMemsetAsync(a.counter, 0, sizeof(unsigned long long), s);
-            if (e != cudaSuccess) return e;
-            kern<<<(unsigned)grid, 128, 0, s>>>((const WideNode*)a.wide, (const uint4*)a.nodes, (const float4*)a.tris, a.num_nodes,
-                                                (const float4*)a.rays, (uint4*)a.hits, (uint32_t)a.n, a.err, (unsigned long long*)a.counter,
-                                                (uint32_t)ch, a.wide_size);
-            return cudaGetLastError();
-        }
         auto pick = [sh](auto k0, auto k8, auto k16, auto k24, auto k32) {
             return sh >= 32 ? k32 : sh >= 24 ? k24 : sh >= 16 ? k16 : sh >= 8 ? k8 : k0;
         };

@@ -55,11 +55,22 @@ PT_HD void apply_point_dev(const float* m, float& x, float& y, float& z) {
     }
 }
 
+template <bool SPLIT>
+PT_HD void load_node(const uint4* p, uint4& a, uint4& b) {
+    if constexpr (SPLIT) {
+        a = ldg(p);
+        b = ldg(p + 1);
+    } else {
+        ldg_node(p, a, b);
+    }
+}
+
 // One instance's bottom-level walk of traverse_two_level (the object-space ray `r`), with the box
 // test fixed for the ray (FAST: box_hits_fast) as in traverse_walk: the two-level 6.5 M-face frame
 // went from 836 to 1070 Msamples/s on a B200.  Returns 0 when the walk ends, 1 when an any-hit ray
-// accepted a face, -1 on a guard failure (res.overflow set).
-template <bool COUNT, int CAP, bool FAST>
+// accepted a face, -1 on a guard failure (res.overflow set).  SPLIT: nodes in two 128-bit loads (code that
+// is not inlined: ptxas 12.9 does not compile the 256-bit load there).
+template <bool COUNT, int CAP, bool FAST, bool SPLIT>
 PT_HD int blas_walk(const TwoLevelView& v, const RayState& r, int mode, uint32_t root, uint32_t fbase, uint32_t pbase,
                     uint32_t ii, bool any, uint32_t* stack, float& min_t, TwoLevelHit& out) {
     TraceResult& res = out.r;
@@ -69,7 +80,7 @@ PT_HD int blas_walk(const TwoLevelView& v, const RayState& r, int mode, uint32_t
         const uint32_t ni = stack[--sp];
         if (ni >= v.num_nodes) { res.overflow = true; return -1; }
         uint4 na, nb;
-        ldg_node(v.nodes + 2 * (size_t)ni, na, nb);
+        load_node<SPLIT>(v.nodes + 2 * (size_t)ni, na, nb);
         if (COUNT) res.nodes++;
         const bool hit = FAST ? box_hits_fast(r, bitsf(na.x), bitsf(na.y), bitsf(na.z), bitsf(na.w), bitsf(nb.x), bitsf(nb.y), min_t)
                               : box_test(r, mode, bitsf(na.x), bitsf(na.y), bitsf(na.z), bitsf(na.w), bitsf(nb.x), bitsf(nb.y), min_t);
@@ -103,7 +114,15 @@ PT_HD int blas_walk(const TwoLevelView& v, const RayState& r, int mode, uint32_t
     return 0;
 }
 
-template <bool COUNT, int CAP = kStackCap>
+// blas_walk for the rays that do not take box_hits_fast (zero direction components and the like), out of
+// line: one copy of the walk instead of two in the frame kernels.
+template <int CAP>
+PT_COLD int blas_walk_general(const TwoLevelView* v, const RayState* r, int mode, uint32_t root, uint32_t fbase, uint32_t pbase, uint32_t ii,
+                              bool any, uint32_t* stack, float* min_t, TwoLevelHit* out) {
+    return blas_walk<false, CAP, false, true>(*v, *r, mode, root, fbase, pbase, ii, any, stack, *min_t, *out);
+}
+
+template <bool COUNT, int CAP = kStackCap, bool SPLIT = false>
 PT_HD TwoLevelHit traverse_two_level(const TwoLevelView& v, float ox, float oy, float oz, float dx, float dy, float dz,
                                      float tmax, bool any) {
     TwoLevelHit out;
@@ -127,7 +146,7 @@ PT_HD TwoLevelHit traverse_two_level(const TwoLevelView& v, float ox, float oy, 
         const uint32_t ti = tstack[--tsp];
         if (ti >= v.top_nodes) { res.overflow = true; return out; }
         uint4 a, b;
-        ldg_node(v.top + 2 * (size_t)ti, a, b);
+        load_node<SPLIT>(v.top + 2 * (size_t)ti, a, b);
         if (COUNT) res.nodes++;
         if (!box_test(wr, wmode, bitsf(a.x), bitsf(a.y), bitsf(a.z), bitsf(a.w), bitsf(b.x), bitsf(b.y), min_t)) continue;
         const uint32_t nf = b.w & 0xFFFFu;
@@ -153,8 +172,20 @@ PT_HD TwoLevelHit traverse_two_level(const TwoLevelView& v, float ox, float oy, 
             RayState r;
             ray_setup(r, lox, loy, loz, ldx, ldy, ldz);
             const int mode = box_mode_for(r, min_t, v.exact_tree);
-            const int st = mode == 0 ? blas_walk<COUNT, CAP, true>(v, r, 0, root, fbase, pbase, ii, any, stack, min_t, out)
-                                     : blas_walk<COUNT, CAP, false>(v, r, mode, root, fbase, pbase, ii, any, stack, min_t, out);
+            int st;
+            if (mode == 0) {
+                st = blas_walk<COUNT, CAP, true, SPLIT>(v, r, 0, root, fbase, pbase, ii, any, stack, min_t, out);
+            } else if constexpr (COUNT || SPLIT) {
+                st = blas_walk<COUNT, CAP, false, SPLIT>(v, r, mode, root, fbase, pbase, ii, any, stack, min_t, out);
+            } else {
+                const TwoLevelView view = v;
+                const RayState ray = r;
+                float far_t = min_t;
+                TwoLevelHit hit = out;
+                st = blas_walk_general<CAP>(&view, &ray, mode, root, fbase, pbase, ii, any, stack, &far_t, &hit);
+                min_t = far_t;
+                out = hit;
+            }
             if (st != 0) return out;
         }
     }

@@ -290,7 +290,7 @@ __global__ void __launch_bounds__(THREADS, 128 * PT_WIDE_BLOCKS / THREADS) wf_wi
         const int live = __popc(~ended);
         if (__popc(leaves) >= (live < PT_WIDE_BATCH ? live : PT_WIDE_BATCH)) {
             if (at_leaf) {
-                wide_faces(k, tris, [&]() { return (const uint4*)p->nodes; }, dir);
+                wide_faces(k, tris, [&]() { return (const uint4*)p->nodes; }, dir, []() { return 0u; });
                 if (k.done) k.cur = kWideDone; else wide_pop(k);
             }
         } else {
@@ -640,19 +640,25 @@ enum PathField : uint32_t {
     kPs, kPsg, kPsb, kPl, kPlg, kPlb,              // throughput, radiance
     kPw, kPwy, kPwz, kPt, kPc, kPcg, kPcb,         // shadow ray: direction, far bound; contribution
     kPbounces, kPslot, kPpixel, kPsample, kPitem, kPtris, kPtrisHi,
-    kPathFields
+    kPathFields,
+    kPinst = kPathFields, kPhitInst, kPentry,      // two-level: the instance being walked, that of the hit, MinT at the entry
+    kPathFieldsTwoLevel
 };
 constexpr uint32_t kIdle = 0, kOnPath = 1, kOnShadow = 2, kToPath = 3, kToShadow = 4, kToEnd = 5;  // lane's ray, or its next
 constexpr uint32_t kRayMask = 7, kPathLambert = 8, kPathPending = 16;                             // and flags of its path
 
-template <int SH>
-__global__ void __launch_bounds__(128, PT_WIDE_PATH_BLOCKS) wf_wide_path_kernel(const WfItem* __restrict__ items,
+// TL: some item may be a two-level scene, whose lanes also cross into and out of instances, PT_WIDE_ENTERS
+// at a time.
+template <int SH, bool TL>
+__global__ void __launch_bounds__(128, TL ? PT_WIDE_TL_BLOCKS : PT_WIDE_PATH_BLOCKS) wf_wide_path_kernel(const WfItem* __restrict__ items,
                                                       const WfSegment* __restrict__ segs, uint32_t nseg, uint32_t count,
                                                       float* __restrict__ radiance, unsigned long long* fetch, uint32_t chunk,
                                                       unsigned long long* rays_traced) {
     const uint32_t lane = threadIdx.x & 31u;
     __shared__ uint2 sstack[SH * 128];
-    __shared__ uint32_t sfield[kPathFields * 128];
+    __shared__ uint32_t sfield[(TL ? kPathFieldsTwoLevel : kPathFields) * 128];
+    bool two = false, inside = true;  // the lane's scene is two-level; its walk is in an instance (or that is none)
+    bool sure = true;                 // a face was accepted in that instance: its box has passed
     const ColdLane cold{sfield + threadIdx.x};
     WideWalkT<kWideStack, SH> k;
     k.stack.base = sstack + threadIdx.x;
@@ -667,9 +673,16 @@ __global__ void __launch_bounds__(128, PT_WIDE_PATH_BLOCKS) wf_wide_path_kernel(
         const bool hit = ended && (state & kRayMask) == kOnPath && k.prim != kPrimNone && ok;
         const uint32_t turns = __ballot_sync(0xFFFFFFFFu, ended && !hit && !(state == kIdle && exhausted));
         const uint32_t hits = __ballot_sync(0xFFFFFFFFu, hit);
-        const uint32_t leaves = __ballot_sync(0xFFFFFFFFu, !ended && (k.cur & kWideLeaf));
+        const bool crosses = TL && !ended && (k.cur == kWideExit || ((k.cur & kWideLeaf) && !inside));
+        const bool at_leaf = !ended && (k.cur & kWideLeaf) && !crosses;
+        const uint32_t crossing = TL ? __ballot_sync(0xFFFFFFFFu, crosses) : 0u;
+        const uint32_t leaves = __ballot_sync(0xFFFFFFFFu, at_leaf);
         const uint32_t walks = __ballot_sync(0xFFFFFFFFu, !(k.cur & kWideLeaf));
-        const int nwalk = __popc(leaves | walks);
+        const int nwalk = __popc(leaves | walks | crossing);
+        // a ray to set up (at one place, behind the steps: the code is long): start is its lane's, and why
+        constexpr uint32_t kNone = 0, kBegin = 1, kEnter = 2, kLeave = 3;
+        uint32_t setup = kNone;
+        F3 o, d;
         if (__popc(turns) >= PT_WIDE_TURNS || (turns && nwalk == 0 && __popc(hits) < PT_WIDE_SHADES)) {
             uint32_t todo = state & kRayMask;
             if (ended && !hit && todo != kIdle) {
@@ -718,8 +731,8 @@ __global__ void __launch_bounds__(128, PT_WIDE_PATH_BLOCKS) wf_wide_path_kernel(
                 const WfSegment sg = segs[find_segment(segs, nseg, slot)];
                 const RenderParams* p = items[sg.item].params;
                 wide = (const WideNode*)p->wide;
+                if (TL) two = p->instances != nullptr;
                 uint32_t pixel, sample;
-                F3 o, d;
                 path_camera(*p, sg.local_begin + (slot - sg.slot_base), pixel, sample, o, d);
                 cold.set3(kPo, o);
                 cold.set3(kPd, d);
@@ -739,12 +752,10 @@ __global__ void __launch_bounds__(128, PT_WIDE_PATH_BLOCKS) wf_wide_path_kernel(
                 state = (state & ~kRayMask) | todo;
                 if (todo == kToPath || todo == kToShadow) {
                     const bool shadow = todo == kToShadow;
-                    const F3 o = cold.f3at(kPo), d = cold.f3at(shadow ? kPw : kPd);
-                    const float tmax = shadow ? cold.f(kPt) : bitsf(0x7F800000u);
-                    const RenderParams* p = items[cold.u(kPitem)].params;
-                    wide_begin(k, o.x, o.y, o.z, d.x, d.y, d.z, tmax, shadow, p->wide_size);
+                    o = cold.f3at(kPo);
+                    d = cold.f3at(shadow ? kPw : kPd);
                     state = (state & ~kRayMask) | (shadow ? kOnShadow : kOnPath);
-                    ok = true;
+                    setup = kBegin;
                 } else {
                     state = kIdle;
                     k.binary = false;
@@ -764,7 +775,12 @@ __global__ void __launch_bounds__(128, PT_WIDE_PATH_BLOCKS) wf_wide_path_kernel(
                 const uint32_t pixel = cold.u(kPpixel), sample = cold.u(kPsample);
                 if (s.bounces == 0 && sample == 0 && it.primary) it.primary[pixel] = k.prim;
                 ShadowReq sh;
-                const bool more = shade_hit(*it.params, s, k.prim, k.leaf, k.u, k.v, k.w, pixel, sample, sh);
+                sh.valid = false;
+                F3 v0, v1, v2;
+                uint32_t mesh;
+                if (TL && two) hit_vertices_two_level(*it.params, k.leaf, cold.u(kPhitInst), v0, v1, v2, mesh);
+                else hit_vertices(*it.params, k.leaf, v0, v1, v2, mesh);
+                const bool more = shade_face(*it.params, s, k.prim, v0, v1, v2, mesh, k.u, k.v, k.w, pixel, sample, sh);
                 cold.set3(kPo, s.o);
                 cold.set3(kPd, s.d);
                 cold.set3(kPs, s.src);
@@ -780,14 +796,51 @@ __global__ void __launch_bounds__(128, PT_WIDE_PATH_BLOCKS) wf_wide_path_kernel(
                     state |= more && !throughput_is_zero(s.src) ? kToPath : kToEnd;
                 }
             }
-        } else if (leaves && __popc(leaves) >= (nwalk < PT_WIDE_BATCH_PATHS ? nwalk : PT_WIDE_BATCH_PATHS)) {
-            if (!ended && (k.cur & kWideLeaf)) {
+        } else if (TL && crossing && (__popc(crossing) >= PT_WIDE_ENTERS || (leaves | walks) == 0)) {
+            if (crosses) {
+                o = cold.f3at(kPo);
+                d = cold.f3at((state & kRayMask) == kOnShadow ? kPw : kPd);
+                if (k.cur == kWideExit) {
+                    inside = false;
+                    wide_pop(k);
+                    if (!(k.cur & kWideLeaf)) setup = kLeave;
+                }
+                if ((k.cur & kWideLeaf) && k.cur != kWideDone) {
+                    cold.set(kPinst, k.cur & kWideIndex);
+                    cold.set(kPentry, k.min_t);
+                    sure = false;
+                    wide_to_object((const DeviceInstance*)items[cold.u(kPitem)].params->instances + (k.cur & kWideIndex), o, d);
+                    setup = kEnter;
+                }
+            }
+        } else if (leaves && __popc(leaves) >= min(__popc(leaves | walks), PT_WIDE_BATCH_PATHS)) {
+            if (at_leaf) {
+                auto instance = [&]() { return (const DeviceInstance*)items[cold.u(kPitem)].params->instances + cold.u(kPinst); };
                 auto dir = [&](float& x, float& y, float& z) {
                     const F3 d = cold.f3at((state & kRayMask) == kOnShadow ? kPw : kPd);
                     x = d.x; y = d.y; z = d.z;
+                    if (TL && two) {
+                        float m[12];
+                        for (int q = 0; q < 12; ++q) m[q] = ldg(instance()->w2o + q);
+                        to_object(m, d.x, d.y, d.z, 0.0f, x, y, z);
+                    }
                 };
-                wide_faces(k, cold.template ptr<float4>(kPtris),
-                           [&]() { return (const uint4*)items[cold.u(kPitem)].params->nodes; }, dir);
+                auto nodes = [&]() {
+                    const uint4* n = (const uint4*)items[cold.u(kPitem)].params->nodes;
+                    return TL && two ? n + 2 * (size_t)ldg(&instance()->node_base) : n;
+                };
+                auto face_base = [&]() { return TL && two ? ldg(&instance()->face_base) : 0u; };
+                if (wide_faces(k, cold.template ptr<float4>(kPtris), nodes, dir, face_base) && TL && two) {
+                    k.prim += ldg(&instance()->prim_base);
+                    cold.set(kPhitInst, cold.u(kPinst));
+                    if (!sure) {
+                        const F3 o = cold.f3at(kPo), d = cold.f3at((state & kRayMask) == kOnShadow ? kPw : kPd);
+                        if (!wide_instance_passes(wide, (const uint4*)items[cold.u(kPitem)].params->top_nodes, cold.u(kPinst), o.x, o.y,
+                                                  o.z, d.x, d.y, d.z, cold.f(kPentry)))
+                            k.binary = k.done = true;
+                        sure = true;
+                    }
+                }
                 if (k.done) k.cur = kWideDone; else wide_pop(k);
             }
         } else if (walks) {
@@ -803,6 +856,28 @@ __global__ void __launch_bounds__(128, PT_WIDE_PATH_BLOCKS) wf_wide_path_kernel(
         } else {
             break;  // every lane idle, no path left
         }
+        if (setup != kNone) {
+            ray_setup(k.r, o.x, o.y, o.z, d.x, d.y, d.z);
+            float size = items[cold.u(kPitem)].params->wide_size;
+            uint4 wi;
+            if (TL && setup == kEnter) {
+                wi = wide_instance(wide, k.cur & kWideIndex);
+                size = bitsf(wi.y);
+            }
+            const bool fits = wide_cut(k.r, k.cut, size);
+            if (setup == kBegin) {
+                const bool shadow = (state & kRayMask) == kOnShadow;
+                wide_start(k, shadow ? cold.f(kPt) : bitsf(0x7F800000u), shadow, fits);
+                ok = true;
+                if (TL) inside = !two;
+            } else if (TL && setup == kEnter) {
+                inside = wide_enter(k, wi.x, fits);
+                if (!inside) {
+                    ok = k.binary;
+                    k.cur = kWideDone;
+                }
+            }
+        }
         // the rays that the records are not for, and those whose MinT rose
         if (k.cur == kWideDone && k.binary) {
             const bool shadow = (state & kRayMask) == kOnShadow;
@@ -810,7 +885,14 @@ __global__ void __launch_bounds__(128, PT_WIDE_PATH_BLOCKS) wf_wide_path_kernel(
             const RenderParams* p = items[cold.u(kPitem)].params;
             const BinaryRay ray{o.x, o.y, o.z, d.x, d.y, d.z, shadow ? cold.f(kPt) : bitsf(0x7F800000u), shadow};
             BinaryHit b;
-            ok = wide_binary_walk((const uint4*)p->nodes, (const float4*)p->tris, p->num_nodes, &ray, &b);
+            if (TL && two) {
+                const TwoLevelView view = two_level_view(*p);
+                uint32_t inst = 0;
+                ok = wide_two_level_walk(&view, &ray, &b, &inst);
+                cold.set(kPhitInst, inst);
+            } else {
+                ok = wide_binary_walk((const uint4*)p->nodes, (const float4*)p->tris, p->num_nodes, &ray, &b);
+            }
             k.prim = b.prim; k.leaf = b.leaf;
             k.u = b.u; k.v = b.v; k.w = b.w;
             k.binary = false;
@@ -1021,13 +1103,14 @@ cudaError_t launch_path_stage(const WfItem* items, const WfSegment* segs, uint32
     return cudaGetLastError();
 }
 
+template <bool TL>
 cudaError_t launch_wide_paths(const WfItem* items, const WfSegment* segs, uint32_t nseg, uint32_t count, float* radiance,
                               unsigned long long* fetch, uint32_t chunk, unsigned long long* rays, cudaStream_t s) {
     constexpr int SH = 16;
     int dev = 0, sms = 0, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, wf_wide_path_kernel<SH>, 128, 0);
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, wf_wide_path_kernel<SH, TL>, 128, 0);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) per_sm = 1;
     uint64_t grid = (uint64_t)sms * per_sm;
@@ -1035,16 +1118,18 @@ cudaError_t launch_wide_paths(const WfItem* items, const WfSegment* segs, uint32
     if (grid > grid_needed) grid = grid_needed ? grid_needed : 1;
     e = cudaMemsetAsync(fetch, 0, sizeof(unsigned long long), s);
     if (e != cudaSuccess) return e;
-    wf_wide_path_kernel<SH><<<(unsigned)grid, 128, 0, s>>>(items, segs, nseg, count, radiance, fetch, chunk, rays);
+    wf_wide_path_kernel<SH, TL><<<(unsigned)grid, 128, 0, s>>>(items, segs, nseg, count, radiance, fetch, chunk, rays);
     return cudaGetLastError();
 }
 
 cudaError_t path_stage(const WfTuning& t, const WfItem* items, const WfSegment* segs, uint32_t nseg, uint32_t count,
                        float* radiance, unsigned long long* fetch, uint32_t chunk, unsigned long long* rays, cudaStream_t s) {
+    if (t.wide)
+        return t.two_level ? launch_wide_paths<true>(items, segs, nseg, count, radiance, fetch, chunk, rays, s)
+                           : launch_wide_paths<false>(items, segs, nseg, count, radiance, fetch, chunk, rays, s);
     if (t.two_level) {  // the top level, the exit marker and the bottom level share the stack: the largest capacity
         return launch_path_stage<64, true>(items, segs, nseg, count, radiance, fetch, chunk, rays, s);
     }
-    if (t.wide) return launch_wide_paths(items, segs, nseg, count, radiance, fetch, chunk, rays, s);
     switch (t.stack_cap) {
         case 24: return launch_path_stage<24, false>(items, segs, nseg, count, radiance, fetch, chunk, rays, s);
         case 32: return launch_path_stage<32, false>(items, segs, nseg, count, radiance, fetch, chunk, rays, s);

@@ -29,6 +29,7 @@
 #pragma once
 
 #include "traverse.cuh"
+#include "two_level.cuh"
 
 namespace pt {
 
@@ -75,11 +76,12 @@ PT_HD bool wide_mark_leaf(const uint4* nodes, uint32_t ni, uint32_t face_base, f
 }
 
 // A slot's reference to binary node `ni` whose second half is `b`; wide_of: the record of each binary
-// node that has one.
-PT_HD uint32_t wide_ref(uint32_t ni, const uint4& b, const uint32_t* wide_of) {
+// node that has one; face_base: face record of the tree's first face.
+PT_HD uint32_t wide_ref(uint32_t ni, const uint4& b, const uint32_t* wide_of, uint32_t face_base) {
     const uint32_t nf = b.w & 0xFFFFu;
     if (nf == 0) return wide_of[ni];
-    return nf < kWideBig && b.z <= kWideIndex ? kWideLeaf | nf << 28 | b.z : kWideLeaf | kWideBig << 28 | ni;
+    return nf < kWideBig && b.z + face_base <= kWideIndex ? kWideLeaf | nf << 28 | (b.z + face_base)
+                                                          : kWideLeaf | kWideBig << 28 | ni;
 }
 
 PT_HD void wide_box(const uint4* nodes, uint32_t i, float lo[3], float hi[3], uint4& b) {
@@ -91,7 +93,7 @@ PT_HD void wide_box(const uint4* nodes, uint32_t i, float lo[3], float hi[3], ui
 
 // Record of binary node `ni`.  Returns whether every box of its slots and of the nodes between lies
 // inside its parent's.
-PT_HD bool wide_make(const uint4* nodes, const uint32_t* wide_of, uint32_t ni, float size, WideNode& w) {
+PT_HD bool wide_make(const uint4* nodes, const uint32_t* wide_of, uint32_t ni, float size, uint32_t face_base, WideNode& w) {
     float lo[4][3], hi[4][3], plo[3], phi[3];
     bool full[4] = {false, false, false, false}, ok = true;
     uint32_t axis[3] = {0, 0, 0};
@@ -106,7 +108,7 @@ PT_HD bool wide_make(const uint4* nodes, const uint32_t* wide_of, uint32_t ni, f
         wide_box(nodes, i, lo[s], hi[s], b);
         inside(lo[s], hi[s], ol, oh);
         full[s] = true;
-        w.ref[s] = wide_ref(i, b, wide_of);
+        w.ref[s] = wide_ref(i, b, wide_of, face_base);
     };
     if ((pb.w & 0xFFFFu) != 0) {  // the root of a tree of one leaf
         slot(0, ni, plo, phi);
@@ -202,45 +204,53 @@ struct WideWalkT {
     WideStack<CAP, SH> stack;
 };
 
-// Starts a walk at record `root`.  Rays with a NaN, a negative or NaN far bound (the binary walk's
-// test of an origin strictly inside a box cannot matter for the others), an origin 2^21 tree sizes
-// away or a direction of extreme length are done at once, `binary` set.
+// Cuts 1/d of a ray (r set up for direction d) for a tree of the given size; false for the rays that the
+// grid test is not proved for: with a NaN, an origin 2^21 tree sizes away or a direction of extreme
+// length.
 //
 // 1/d is cut at 2^50 times the least of the three.  A plane ahead of the origin is then met sooner, so
 // near only falls.  The far plane lies a 32nd of a grid step, at least 2^-27 of the tree's size, beyond
 // the box: a ray whose origin is not past the box meets it no sooner than 2^23 * size * least, and
 // every box of the tree ends before 2 (1 + 2^21) * size * least on the axis of the least 1/d.
-template <int CAP, int SH>
-PT_HD void wide_begin(WideWalkT<CAP, SH>& k, float ox, float oy, float oz, float dx, float dy, float dz, float tmax, bool any,
-                      float size, uint32_t root = 0) {
-    ray_setup(k.r, ox, oy, oz, dx, dy, dz);
-    const float ax = fabs_(k.r.ix), ay = fabs_(k.r.iy), az = fabs_(k.r.iz);
+PT_HD bool wide_cut(RayState& r, bool& cut, float size) {
+    const float ax = fabs_(r.ix), ay = fabs_(r.iy), az = fabs_(r.iz);
     const float least = fminf(fminf(ax, ay), az), most = fmaxf(fmaxf(ax, ay), az), top = fmul(least, kWideSlope);
-    const float far_o = fmaxf(fmaxf(fabs_(ox), fabs_(oy)), fabs_(oz));
+    const float far_o = fmaxf(fmaxf(fabs_(r.ox), fabs_(r.oy)), fabs_(r.oz));
     const float scale = fmul(least, size);
-    const bool fits = tmax >= 0.f && scale >= kWideScaleMin && scale <= kWideScaleMax && top < bitsf(0x7F800000u) &&
-                      far_o <= fmul(kWideFar, size) && ax == ax && ay == ay && az == az && ox == ox && oy == oy && oz == oz;
-    k.cut = !(most <= top);
-    if (k.cut) {
-        k.r.ix = ax > top ? bitsf(fbits(top) | (fbits(k.r.ix) & 0x80000000u)) : k.r.ix;
-        k.r.iy = ay > top ? bitsf(fbits(top) | (fbits(k.r.iy) & 0x80000000u)) : k.r.iy;
-        k.r.iz = az > top ? bitsf(fbits(top) | (fbits(k.r.iz) & 0x80000000u)) : k.r.iz;
+    const bool fits = scale >= kWideScaleMin && scale <= kWideScaleMax && top < bitsf(0x7F800000u) &&
+                      far_o <= fmul(kWideFar, size) && ax == ax && ay == ay && az == az && r.ox == r.ox && r.oy == r.oy && r.oz == r.oz;
+    cut = !(most <= top);
+    if (cut) {
+        r.ix = ax > top ? bitsf(fbits(top) | (fbits(r.ix) & 0x80000000u)) : r.ix;
+        r.iy = ay > top ? bitsf(fbits(top) | (fbits(r.iy) & 0x80000000u)) : r.iy;
+        r.iz = az > top ? bitsf(fbits(top) | (fbits(r.iz) & 0x80000000u)) : r.iz;
     }
+    return fits;
+}
+
+// Starts the walk of the ray in k.r at record 0.  Rays that wide_cut refused (fits), and those with a
+// negative or NaN far bound (the binary walk's test of an origin strictly inside a box cannot matter
+// for the others), are done at once, `binary` set.
+template <int CAP, int SH>
+PT_HD void wide_start(WideWalkT<CAP, SH>& k, float tmax, bool any, bool fits) {
+    fits = fits && tmax >= 0.f;
     k.min_t = tmax;
     k.prim = kPrimNone;
     k.leaf = kPrimNone;
     k.u = k.v = k.w = 0.f;
     k.any = any;
     k.done = k.binary = !fits;
-    k.cur = fits ? root : kWideDone;
+    k.cur = fits ? 0u : kWideDone;
     k.sp = 0;
 }
 
-#ifdef __CUDACC__
-#define PT_COLD inline __host__ __device__ __noinline__
-#else
-#define PT_COLD inline
-#endif
+template <int CAP, int SH>
+PT_HD void wide_begin(WideWalkT<CAP, SH>& k, float ox, float oy, float oz, float dx, float dy, float dz, float tmax, bool any,
+                      float size) {
+    ray_setup(k.r, ox, oy, oz, dx, dy, dz);
+    const bool fits = wide_cut(k.r, k.cut, size);
+    wide_start(k, tmax, any, fits);
+}
 
 // The binary walk of a whole ray, out of line: the hit in *out, false on a guard failure.  Nodes come in
 // two 128-bit loads: ptxas 12.9 does not compile the 256-bit load in a function that is not inlined.
@@ -401,14 +411,15 @@ PT_HD bool wide_leaf_passes(const K& k, float4 q0, float4 q1, float4 q2, const N
 
 // The faces of leaf k.cur in leaf order, as the binary walk tests them; sets k.done when the walk ends
 // here (an any-hit ray accepted a face, or MinT rose and `binary` is set).  `nodes` gives the binary nodes,
-// which only large leaves and boxes to be tested exactly need.
-template <int CAP, int SH, class Nodes, class Dir>
-PT_HD void wide_faces(WideWalkT<CAP, SH>& k, const float4* __restrict__ tris, const Nodes& nodes, const Dir& dir) {
+// which only large leaves and boxes to be tested exactly need, `face_base` the face record of the tree's first
+// face (large leaves).  Returns whether a face was accepted.
+template <int CAP, int SH, class Nodes, class Dir, class Base>
+PT_HD bool wide_faces(WideWalkT<CAP, SH>& k, const float4* __restrict__ tris, const Nodes& nodes, const Dir& dir, const Base& face_base) {
     uint32_t at = k.cur & kWideIndex, n = (k.cur >> 28) & 7u;
     if (n == kWideBig) {
         uint4 a, b;
         ldg_node(nodes() + 2 * (size_t)at, a, b);
-        at = b.z;
+        at = b.z + face_base();
         n = b.w & 0xFFFFu;
     }
     const float before = k.min_t;
@@ -419,17 +430,81 @@ PT_HD void wide_faces(WideWalkT<CAP, SH>& k, const float4* __restrict__ tris, co
         float t, u, v, w;
         if (wald(k.r, q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w, q2.x, k.min_t, t, u, v, w)) {
             if (!passes) {
-                if (!wide_leaf_passes(k, q0, q1, q2, nodes, before, dir)) return;
+                if (!wide_leaf_passes(k, q0, q1, q2, nodes, before, dir)) return false;
                 passes = true;
             }
-            if (t > k.min_t && !k.any) { k.binary = k.done = true; return; }
+            if (t > k.min_t && !k.any) { k.binary = k.done = true; return false; }
             k.min_t = t;
             k.prim = fbits(q2.y);
             k.leaf = at + j;
             k.u = u; k.v = v; k.w = w;
-            if (k.any) { k.done = true; return; }
+            if (k.any) { k.done = true; return true; }
         }
     }
+    return passes;
+}
+
+// ---- two-level scenes -------------------------------------------------------------------------------
+//
+// The top-level tree's records come first in the array, then those of every geometry's tree; a table of
+// the instances lies before record 0 (WideInstance, pt_internal.h).  A walk starts in world space; at a
+// top-level leaf the ray is carried into its instance's object space, an exit marker is pushed and the
+// walk goes on at the geometry's first record.  Boxes and faces are tested in traverse_two_level's order;
+// the instance's own box is tested exactly, at the MinT of the entry, before the first face accepted in
+// it counts (wide_instance_passes; where it fails, traverse_two_level takes the whole ray).  The world
+// ray is set up again only when a top-level record follows an exit: most often another instance does, or
+// the walk's end.
+constexpr uint32_t kWideExit = 0xFFFFFFFEu;  // exit marker (its leaf bit set: no record)
+
+// WideInstance of instance ii: {root, size, node, 0}.
+PT_HD uint4 wide_instance(const WideNode* wide, uint32_t ii) { return ldg((const uint4*)wide - 1 - ii); }
+
+// A world ray in the object space of an instance.
+template <class V>
+PT_HD void wide_to_object(const DeviceInstance* inst, V& o, V& d) {
+    const float4* w2o = (const float4*)inst->w2o;
+    const float4 m0 = ldg(w2o), m1 = ldg(w2o + 1), m2 = ldg(w2o + 2);
+    const float m[12] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w, m2.x, m2.y, m2.z, m2.w};
+    const V wo = o, wd = d;
+    to_object(m, wo.x, wo.y, wo.z, 1.0f, o.x, o.y, o.z);
+    to_object(m, wd.x, wd.y, wd.z, 0.0f, d.x, d.y, d.z);
+}
+
+// Enters the instance whose tree starts at record root, with its object ray in k.r.  False when that ray is
+// none for the records (wide_cut's fits; done and `binary` set) or the stack is full (done set).
+template <int CAP, int SH>
+PT_HD bool wide_enter(WideWalkT<CAP, SH>& k, uint32_t root, bool fits) {
+    if (!fits || k.sp >= CAP) {
+        k.done = true;
+        k.binary = !fits;
+        return false;
+    }
+    k.stack.put(k.sp++, kWideExit, 0.f);
+    k.cur = root;
+    return true;
+}
+
+// Whether the box of instance ii passes for world ray o, d at far bound min_t.
+PT_HD bool wide_instance_passes(const WideNode* __restrict__ wide, const uint4* __restrict__ top, uint32_t ii, float ox, float oy, float oz,
+                                float dx, float dy, float dz, float min_t) {
+    const uint4* q = top + 2 * (size_t)wide_instance(wide, ii).z;
+    const uint4 a = ldg(q), b = ldg(q + 1);
+    RayState r;
+    r.ox = ox; r.oy = oy; r.oz = oz;
+    r.ix = frcp(dx); r.iy = frcp(dy); r.iz = frcp(dz);
+    return box_hits(r, bitsf(a.x), bitsf(a.y), bitsf(a.z), bitsf(a.w), bitsf(b.x), bitsf(b.y), min_t, false);
+}
+
+// The whole ray by traverse_two_level, out of line: the hit in *out, its instance in *inst; false on a guard
+// failure.
+PT_COLD bool wide_two_level_walk(const TwoLevelView* v, const BinaryRay* ray, BinaryHit* out, uint32_t* inst) {
+    const TwoLevelHit h = traverse_two_level<false, kStackCap, true>(*v, ray->ox, ray->oy, ray->oz, ray->dx, ray->dy, ray->dz, ray->tmax,
+                                                                     ray->any);
+    out->t = h.r.t;
+    out->u = h.r.u; out->v = h.r.v; out->w = h.r.w;
+    out->prim = h.r.prim; out->leaf = h.r.leaf;
+    *inst = h.inst;
+    return !h.r.overflow;
 }
 
 }  // namespace pt

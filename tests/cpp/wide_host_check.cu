@@ -38,7 +38,7 @@ static bool walk(WideWalkT<CAP, SH>& k, const std::vector<WideNode>& wide, const
     while (k.cur != kWideDone) {
         ++steps;
         if (k.cur & kWideLeaf) {
-            wide_faces(k, tris.data(), [&]() { return nodes.data(); }, dir);
+            wide_faces(k, tris.data(), [&]() { return nodes.data(); }, dir, []() { return 0u; });
             if (k.done) break;
         } else if (!wide_visit(k, wide.data())) {
             return false;
@@ -73,7 +73,7 @@ int main(int argc, char** argv) {
         const bool leaf = (nodes[2 * (size_t)i + 1].w & 0xFFFFu) != 0;
         if (leaf) nested = wide_mark_leaf(nodes.data(), i, 0, tris.data()) && nested;
         if (i == 0 || (!leaf && (depth[i] & 1u) == 0))
-            nested = wide_make(nodes.data(), wide_of.data(), i, size, wide[wide_of[i]]) && nested;
+            nested = wide_make(nodes.data(), wide_of.data(), i, size, 0, wide[wide_of[i]]) && nested;
     }
     if (!nested) {
         std::fprintf(stderr, "a box does not lie inside its parent's\n");

@@ -102,3 +102,34 @@ def test_batches_with_and_without_records(cuda_device, pipeline, threads):
         b.close()
     for s in scenes:
         s.close()
+
+
+def instances(name):
+    if name == "one":
+        return W.instanced_scene(level=2, instances=1)[0][1:2]
+    if name == "forty":
+        return W.instanced_scene(level=3, instances=40)[0]
+    if name == "leaves":  # geometries of one leaf, one of them large, under identity and other transforms
+        m = [copies(20, 0), grid(3)]
+        o = W.instanced_scene(level=2, instances=3)[0][1].object_to_world
+        return m + [pb.Mesh(m[0].x, m[0].y, m[0].z, m[0].faces, object_to_world=o)]
+    return W.instanced_scene(level=5, instances=5)[0]
+
+
+@pytest.mark.parametrize("name", ["one", "five", "forty", "leaves"])
+def test_two_level_queries_match_the_counted_walk(cuda_device, name):
+    s = pb.Scene(instances(name), two_level=True)
+    for n in (1, 33, 2369, 100_003):
+        same_hits(s, np.concatenate([edge_case_rays(n, 5), axis_rays(n, 6), slanted_rays(n, 7)]))
+    s.close()
+
+
+@pytest.mark.parametrize("name", ["one", "five", "forty", "leaves"])
+def test_two_level_frames_match_the_fused_walk(cuda_device, name):
+    s = pb.Scene(instances(name), env=(51.0,) * 3, two_level=True)
+    for size, spp in (((1, 1), 1), ((33, 33), 3), ((130, 67), 2)):
+        args = (size[0], size[1], spp, 5, AXIS_CAMERA, 9)
+        film, prim = pb.render(s, *args, flags=pb.RENDER_NEE | pb.RENDER_FUSED)
+        got, gprim = pb.render(s, *args, flags=pb.RENDER_NEE | pb.RENDER_PERSISTENT)
+        assert got.tobytes() == film.tobytes() and gprim.tobytes() == prim.tobytes()
+    s.close()
