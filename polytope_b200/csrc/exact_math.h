@@ -319,12 +319,7 @@ float f64_diff_emulated(float a, float b, float c, float d) {
 // ------------------------------------------------------------------------------------------------
 // Counter-based RNG: Philox4x32-10 (Salmon, Moraes, Dror, Shaw, SC'11).
 PT_HD void philox4x32(uint32_t c[4], uint32_t k0, uint32_t k1) {
-#ifdef PT_PHILOX_UNROLL
-    constexpr int kUnroll = PT_PHILOX_UNROLL;
-#else
-    constexpr int kUnroll = 10;
-#endif
-#pragma unroll kUnroll
+#pragma unroll
     for (int r = 0; r < 10; ++r) {
         const uint64_t p0 = (uint64_t)0xD2511F53u * c[0];
         const uint64_t p1 = (uint64_t)0xCD9E8D57u * c[2];

@@ -146,6 +146,7 @@ struct SceneDev {
 
 struct pt_scene {
     pt::SceneDev dev;
+    void* memory = nullptr;  // the allocation that holds all of dev, the error flag and the ray counters
     uint32_t num_nodes = 0;
     uint32_t num_prims = 0;
     uint32_t num_meshes = 0;
@@ -163,7 +164,7 @@ struct pt_scene {
     void* dev_in = nullptr;
     void* dev_out = nullptr;
     size_t staging_rays = 0;
-    void* streams[4] = {};  // host-pointer traces: copies in, two kernel streams, copies out
+    void* streams[8] = {};  // host-pointer traces: copies in, two kernel streams, copies out (of pageable arrays: one a worker)
     void* events[16] = {};
     // device ints set when a kernel hits a guard: err_flag by the asynchronous (device-memory)
     // calls, cleared when pt_scene_status reports it; trace_err by the host-memory pt_trace call
@@ -171,7 +172,6 @@ struct pt_scene {
     void* err_flag = nullptr;
     void* trace_err = nullptr;
     bool two_level = false;  // made by pt_scene_create_two_level
-    void* wide_base = nullptr;  // allocation that holds dev.wide
     float wide_size = 0.f;      // largest coordinate of the (top-level) tree's boxes
     bool nan_boxes = false;  // some tree box holds a NaN (every ray then takes the exact box test)
     // ray counters of the persistent trace kernel: one per launch in flight, taken round-robin

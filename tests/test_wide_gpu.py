@@ -133,3 +133,31 @@ def test_two_level_frames_match_the_fused_walk(cuda_device, name):
         got, gprim = pb.render(s, *args, flags=pb.RENDER_NEE | pb.RENDER_PERSISTENT)
         assert got.tobytes() == film.tobytes() and gprim.tobytes() == prim.tobytes()
     s.close()
+
+
+@pytest.mark.parametrize("n", [65_535, 65_536, 65_537, 131_073, 4_300_007])
+def test_host_arrays_around_the_worker_threshold(cuda_device, n):
+    """Pageable arrays in parallel from 65,536 rays on; rays or hits in pinned memory beside them."""
+    import torch
+    s = pb.Scene(W.small_scene(3)[0])
+    rays = np.resize(edge_case_rays(50_000, 11), n)
+    ref, _, _ = s.intersect(rays, counts=True)
+    assert s.intersect(rays).tobytes() == ref.tobytes()
+    pinned_rays = torch.empty(32 * n, dtype=torch.uint8).pin_memory().numpy().view(pb.RAY_DTYPE)
+    pinned_hits = torch.empty(16 * n, dtype=torch.uint8).pin_memory().numpy().view(pb.HIT_DTYPE)
+    pinned_rays[:] = rays
+    assert s.intersect(pinned_rays).tobytes() == ref.tobytes()
+    s.intersect(rays, pinned_hits)
+    assert pinned_hits.tobytes() == ref.tobytes()
+    s.close()
+
+
+def test_host_arrays_from_several_threads(cuda_device):
+    from concurrent.futures import ThreadPoolExecutor
+    s = pb.Scene(W.small_scene(4)[0])
+    sets = [edge_case_rays(100_000 + 7 * k, k) for k in range(6)]
+    ref = [s.intersect(r, counts=True)[0].tobytes() for r in sets]
+    with ThreadPoolExecutor(6) as ex:
+        for _ in range(3):
+            assert [h.tobytes() for h in ex.map(s.intersect, sets)] == ref
+    s.close()
