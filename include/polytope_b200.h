@@ -391,10 +391,11 @@ typedef struct pt_batch_item {
  *                          takes the next pixel of any render (wave_pixels: pixels per launch).
  *   PT_PIPELINE_WAVEFRONT: waves of paths of all renders; per bounce a persistent extend kernel,
  *                          a shade kernel appending to ray / shadow queues, a persistent shadow
- *                          kernel (wave_pixels: paths per wave).
+ *                          kernel (wave_pixels: paths per wave).  Waves of few paths (131,072 a
+ *                          bounce at most) run as PT_PIPELINE_PATHS when all scenes have
+ *                          four-wide records.
  *   PT_PIPELINE_PATHS:     waves of paths of all renders as in PT_PIPELINE_WAVEFRONT, but one
- *                          thread runs a whole path (pt_render's fused kernel over several
- *                          renders at once; wave_pixels: paths per wave). */
+ *                          persistent kernel runs whole paths (wave_pixels: paths per wave). */
 #define PT_PIPELINE_FUSED     0u
 #define PT_PIPELINE_WAVEFRONT 1u
 #define PT_PIPELINE_PATHS     2u

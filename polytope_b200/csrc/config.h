@@ -93,3 +93,14 @@
 #ifndef PT_WIDE_ENTERS
 #define PT_WIDE_ENTERS 8
 #endif
+
+// Paths per bounce up to which a wave over four-wide records runs as whole paths in the persistent path
+// kernel instead of bounce by bounce: a bounce costs six launches, each as long as its slowest ray, which
+// few paths don't cover.  Bounce by bounce / whole paths on a B200 (ms; eight scenes of 20 k faces each):
+// depth 0 (one bounce), 131 k paths 0.13 / 0.13, 524 k 0.26 / 0.27; depth 2, 131 k 0.65 / 0.48, 393 k 0.93 /
+// 0.90, 786 k 1.44 / 1.49; depth 6, 131 k 1.04 / 0.57, 917 k 2.16 / 1.95; depth 12, 131 k 3.11 / 1.24, 2.1 M
+// 7.66 / 6.89.  Scenes of 1 k faces gain more, of 500 k faces the same; far above the line the waves are
+// 8 % ahead (24 uneven renders, 24.5 against 26.3).
+#ifndef PT_WIDE_WAVE_PATHS
+#define PT_WIDE_WAVE_PATHS (1u << 17)
+#endif

@@ -1205,7 +1205,8 @@ cudaError_t wf_launch_wave(const WfItem* d_items, const WfSegment* d_segments, c
     if (w.count == 0) return cudaSuccess;
     if (w.count > ws.capacity) return cudaErrorInvalidValue;
     if (!t.paths && !ws.ray_o) return cudaErrorInvalidValue;  // state carved for the path kernel only
-    cudaError_t e = t.paths ? path_stage(t, d_items, d_segments + w.seg_begin, w.seg_count, w.count,
+    const bool paths = t.paths || (t.wide && w.count <= (uint64_t)w.bounces * PT_WIDE_WAVE_PATHS);
+    cudaError_t e = paths ? path_stage(t, d_items, d_segments + w.seg_begin, w.seg_count, w.count,
                                          ws.radiance, (unsigned long long*)(ws.counters + 4), t.queue_chunk, rays_traced, s)
                             : bounce_stages(d_items, d_segments, w, ws, t, rays_traced, s);
     if (e != cudaSuccess) return e;

@@ -74,7 +74,7 @@ struct WfTuning {
     uint32_t threads_per_block = 128;  // extend / shadow kernels
     uint32_t queue_chunk = 64;         // rays a warp takes per fetch in the persistent kernels
     int stack_cap = 64;                // traversal stack entries
-    bool paths = false;                // one thread per whole path instead of per-bounce kernels
+    bool paths = false;                // whole paths in one kernel instead of per-bounce kernels
     bool two_level = false;            // (paths only) some item is a two-level scene
     bool wide = false;                 // every item has four-wide records
 };
@@ -107,8 +107,9 @@ void wf_add_wave(WfPlan& plan, const std::vector<WfSegment>& segs, const std::ve
 void wf_plan_all(WfPlan& plan, const std::vector<uint32_t>& npix, const std::vector<uint32_t>& spp,
                  const std::vector<uint32_t>& max_depth, uint64_t wave_paths);
 
-// Enqueues one wave on `s` (per-bounce kernels, or with t.paths one kernel running whole paths).  d_items / d_segments / d_resolve / d_finish are device copies of the
-// plan's tables (the wave's ranges index into them).
+// Enqueues one wave on `s`: per-bounce kernels, or one kernel running whole paths with t.paths and for
+// waves of few paths over four-wide records (PT_WIDE_WAVE_PATHS).  d_items / d_segments / d_resolve /
+// d_finish are device copies of the plan's tables (the wave's ranges index into them).
 cudaError_t wf_launch_wave(const WfItem* d_items, const WfSegment* d_segments, const WfPixels* d_resolve,
                            const WfPixels* d_finish, const WfWave& w, const WfState& ws, const WfTuning& t,
                            unsigned long long* rays_traced, cudaStream_t s);

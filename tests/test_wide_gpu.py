@@ -104,6 +104,26 @@ def test_batches_with_and_without_records(cuda_device, pipeline, threads):
         s.close()
 
 
+@pytest.mark.parametrize("threads", [64, 128, 256])
+@pytest.mark.parametrize("width, depth, spp, wave", [(512, 0, 1, 0), (513, 0, 1, 0), (512, 2, 3, 0), (513, 2, 3, 0), (515, 0, 3, 256 * 600)])
+def test_waves_around_the_whole_path_limit(cuda_device, threads, width, depth, spp, wave):
+    """Waves of up to 131,072 paths a bounce run as whole paths, larger ones bounce by bounce; the last
+    case has two of the one kind and one of the other in a batch."""
+    s = pb.Scene(scene("boxes"), env=(51.0,) * 3)
+    t = pb.default_tuning()
+    t.pipeline, t.threads_per_block, t.wave_pixels = pb.PIPELINE_WAVEFRONT, threads, wave
+    rd = pb.render_desc(width, 256, spp, depth, AXIS_CAMERA, 4, pb.RENDER_NEE)
+    film, prim = pb.render(s, width, 256, spp, depth, AXIS_CAMERA, 4, pb.RENDER_NEE | pb.RENDER_FUSED)
+    b = pb.Batch([(s, rd)], t)
+    b.run()
+    got, gprim = b.output(0)
+    assert got.tobytes() == film.tobytes() and gprim.tobytes() == prim.tobytes()
+    b.close()
+    got, gprim = pb.render(s, width, 256, spp, depth, AXIS_CAMERA, 4, pb.RENDER_NEE | pb.RENDER_WAVEFRONT)
+    assert got.tobytes() == film.tobytes() and gprim.tobytes() == prim.tobytes()
+    s.close()
+
+
 def instances(name):
     if name == "one":
         return W.instanced_scene(level=2, instances=1)[0][1:2]
