@@ -59,6 +59,19 @@
 #ifndef PT_WIDE_STEPS
 #define PT_WIDE_STEPS 4
 #endif
+// A warp that has no more rays to take is as slow as its slowest lane: there fewer lanes wait for faces to
+// be tested, and a lane may test a second leaf at once.  1 k rays 26.9 -> 25.6 us, 100 k on box faces 97 ->
+// 95, 1 M occlusion rays 565 -> 517, 16.7 M rays 5187 -> 5128 (the path kernel's 1920x1080x16 frame, a
+// second leaf only: 9.24 -> 9.12 ms).  With all rays a second leaf costs 7 % on 16.7 M.  A batch of 16 there
+// gives 25.7 / 92.5 / 540 / 5119, of 4 27.4 / 95.7 / 505 / 5161; four leaves 25.7 / 93.1 / 543 / 5135; 8
+// visits between votes 25.5 / 91.5 / 543 / 5147 at 16.  Two-level queries are 1 % slower with it and keep
+// the constants above.
+#ifndef PT_WIDE_LAST_BATCH
+#define PT_WIDE_LAST_BATCH 8
+#endif
+#ifndef PT_WIDE_LAST_LEAVES
+#define PT_WIDE_LAST_LEAVES 2
+#endif
 
 // The same for the persistent path kernel (wf_wide_path_kernel), with the lanes that must have a ray to
 // end or start, or a hit to shade, before those steps run.  Measured on a B200 (ms; 1920x1080x16 frame

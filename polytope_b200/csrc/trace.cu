@@ -290,9 +290,9 @@ __global__ void __launch_bounds__(128, TL ? PT_WIDE_TL_BLOCKS : PT_WIDE_BLOCKS) 
             continue;
         }
         const bool crosses = TL && k.cur != kWideDone && (k.cur == kWideExit || ((k.cur & kWideLeaf) && !inside));
-        const bool at_leaf = k.cur != kWideDone && (k.cur & kWideLeaf) && !crosses;
-        const uint32_t leaves = __ballot_sync(0xFFFFFFFFu, at_leaf);
-        uint32_t live = __popc(~ended);
+        auto at_face = [&]() { return (k.cur & kWideLeaf) && k.cur < kWideExit && (!TL || inside); };
+        const uint32_t leaves = __ballot_sync(0xFFFFFFFFu, at_face());
+        int live = __popc(~ended);
         if constexpr (TL) {
             const uint32_t crossing = __ballot_sync(0xFFFFFFFFu, crosses);
             live -= __popc(crossing);  // the lanes that walk
@@ -329,8 +329,10 @@ __global__ void __launch_bounds__(128, TL ? PT_WIDE_TL_BLOCKS : PT_WIDE_BLOCKS) 
                 continue;
             }
         }
-        if (__popc(leaves) >= (live < PT_WIDE_BATCH ? live : PT_WIDE_BATCH)) {
-            if (at_leaf) {
+        const bool last = !TL && exhausted;  // the warp's last rays
+        if (__popc(leaves) >= min(live, last ? PT_WIDE_LAST_BATCH : PT_WIDE_BATCH)) {
+#pragma unroll 1
+            for (int step = 0; step < (last ? PT_WIDE_LAST_LEAVES : 1) && at_face(); ++step) {
                 if constexpr (TL) {
                     const DeviceInstance* in = inst + sinst[threadIdx.x];
                     if (wide_faces(k, tris, [&]() { return nodes + 2 * (size_t)ldg(&in->node_base); }, dir,

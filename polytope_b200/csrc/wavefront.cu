@@ -288,8 +288,9 @@ __global__ void __launch_bounds__(THREADS, 128 * PT_WIDE_BLOCKS / THREADS) wf_wi
         const bool at_leaf = k.cur != kWideDone && (k.cur & kWideLeaf);
         const uint32_t leaves = __ballot_sync(0xFFFFFFFFu, at_leaf);
         const int live = __popc(~ended);
-        if (__popc(leaves) >= (live < PT_WIDE_BATCH ? live : PT_WIDE_BATCH)) {
-            if (at_leaf) {
+        if (__popc(leaves) >= min(live, exhausted ? PT_WIDE_LAST_BATCH : PT_WIDE_BATCH)) {
+#pragma unroll 1
+            for (int step = 0; step < (exhausted ? PT_WIDE_LAST_LEAVES : 1) && (k.cur & kWideLeaf) && k.cur != kWideDone; ++step) {
                 wide_faces(k, tris, [&]() { return (const uint4*)p->nodes; }, dir, []() { return 0u; });
                 if (k.done) k.cur = kWideDone; else wide_pop(k);
             }
@@ -814,7 +815,8 @@ __global__ void __launch_bounds__(128, TL ? PT_WIDE_TL_BLOCKS : PT_WIDE_PATH_BLO
                 }
             }
         } else if (leaves && __popc(leaves) >= min(__popc(leaves | walks), PT_WIDE_BATCH_PATHS)) {
-            if (at_leaf) {
+#pragma unroll 1
+            for (int step = 0; step < (exhausted ? PT_WIDE_LAST_LEAVES : 1) && (k.cur & kWideLeaf) && k.cur < kWideExit && (!TL || inside); ++step) {
                 auto instance = [&]() { return (const DeviceInstance*)items[cold.u(kPitem)].params->instances + cold.u(kPinst); };
                 auto dir = [&](float& x, float& y, float& z) {
                     const F3 d = cold.f3at((state & kRayMask) == kOnShadow ? kPw : kPd);
