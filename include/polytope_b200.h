@@ -161,7 +161,8 @@ typedef struct pt_scene_info {
     uint32_t num_prims;
     uint32_t num_meshes;
     uint32_t max_depth;            /* deepest node level (root = 0)                           */
-    uint64_t device_bytes;         /* device memory held by the handle                        */
+    uint64_t device_bytes;         /* nodes, faces and the other arrays of the description (the
+                                    * four-wide records, about a quarter more, are not counted)*/
 } pt_scene_info;
 int pt_scene_get_info(const pt_scene *scene, pt_scene_info *info);
 
@@ -206,7 +207,7 @@ int pt_trace_counted(pt_scene *scene, const pt_ray *rays, uint64_t n, pt_hit *hi
 
 /* Launch shape of the ray-query kernel (per scene).  shared_stack: traversal-stack entries per
  * lane kept in shared memory (0, 8, 16, 24 or 32; the rest stays in local memory); queue_chunk: rays a
- * warp takes per fetch (multiple of 32).  Results do not depend on it. */
+ * warp takes per fetch (multiple of 32; twice that while there are plenty, fewer at the end).  Results do not depend on it. */
 typedef struct pt_trace_tuning {
     uint32_t shared_stack;
     uint32_t queue_chunk;

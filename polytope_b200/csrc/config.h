@@ -76,7 +76,8 @@
 // The same for the persistent path kernel (wf_wide_path_kernel), with the lanes that must have a ray to
 // end or start, or a hit to shade, before those steps run.  Measured on a B200 (ms; 1920x1080x16 frame
 // of 3.9 M faces / 641x479x4 frame of 20 k box faces / 24 served requests), before the binary walk's
-// kernel and after: 12.9 / 3.35 / 9.0 -> 9.4 / 2.7 / 6.1.  One visit between votes 9.5 / 3.0 / 6.5; 4 blocks
+// kernel and after: 12.9 / 3.35 / 9.0 -> 9.4 / 2.7 / 6.1 (9.1 / 2.5 / 5.9 with the last paths handed out in
+// small lots, wide_take).  One visit between votes 9.5 / 3.0 / 6.5; 4 blocks
 // 10.2 / 2.85 / 6.2, 6 blocks 9.4 / 2.7 / 6.1 (one visit: 11.1 / 3.3 / 7.1); turns from 4 or 16 lanes on
 // within 2 %, shading from 10 or 24 lanes on 3 to 7 % slower on the first.
 #ifndef PT_WIDE_PATH_BLOCKS

@@ -1,13 +1,15 @@
 // render.cu -- the render call (TileRunner::Run + AbstractRunner::Trace + PathTraceIntegrator)
 // as sm_100a kernels.  Paths are numbered sample-major (path = sample * W*H + pixel) and rendered
 // in waves.  Three pipelines compute identical results:
-//   * persistent (the default): one persistent path kernel per wave (wavefront.cu wf_path_kernel)
-//                whose lanes take the next path as soon as theirs ends;
+//   * persistent (the default): one persistent path kernel per wave (wavefront.cu wf_wide_path_kernel,
+//                wf_path_kernel for trees without four-wide records) whose lanes take the next path as
+//                soon as theirs ends;
 //   * fused:     one thread runs a whole path (camera ray, bounces, shadow rays), one launch per
-//                wave (path_kernel below; the default for two-level scenes);
+//                wave (path_wide_kernel, path_kernel below; the default for two-level scenes);
 //   * wavefront: per bounce an extend kernel (closest hit) over a compacted queue, a shade kernel
 //                that appends the next rays and the shadow rays to queues with warp-vote
-//                compaction and one atomic per warp, and a shadow kernel (any hit).
+//                compaction and one atomic per warp, and a shadow kernel (any hit); waves of few paths
+//                over records run as the persistent pipeline's.
 // Each way a resolve kernel then adds each pixel's samples to the film in sample order (the
 // order of BoxFilter::Output's sum, BoxFilter.cpp:54-71), so the film is deterministic and equal
 // to the CPU oracle's bit for bit.
@@ -283,7 +285,7 @@ int enqueue_frame(pt_scene* s, const pt_render_desc* desc, float* rgb_d, uint32_
     // (the wave engine runs both the queue-based kernels and the persistent path kernel).
     // two-level scenes default to the fused kernel: coherent paths cross their instances together there,
     // while the persistent kernel's crossings interrupt its steps (1280x720x8 frame of five instances:
-    // 4.4 ms fused, 5.9 persistent, 8.0 over the binary trees)
+    // 4.3 ms fused, 5.4 persistent, 14.5 over the binary trees)
     const bool fused = (desc->flags & PT_RENDER_FUSED) != 0 || (s->two_level && !(desc->flags & PT_RENDER_PERSISTENT));
     const bool persistent = !fused && (desc->flags & PT_RENDER_WAVEFRONT) == 0;
     const bool wavefront = !fused;

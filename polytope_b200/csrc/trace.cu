@@ -1,8 +1,9 @@
 // trace.cu -- ray-query kernels (Scene::intersect replacement) for sm_100a.
 //
-// One thread per ray, reference-order traversal (traverse.cuh).  Rays and hits stream through
-// HBM once (32 B in, 16 B out per ray); nodes and faces are read with 128-bit read-only loads and
-// stay resident in the 126 MB L2 for scenes up to a few million faces.
+// Queries of scenes that have four-wide records (wide.cuh) run in trace_wide_kernel; counted queries and
+// trees without records walk the binary nodes in the reference's order (traverse.cuh).  Rays and hits
+// stream through HBM once (32 B in, 16 B out per ray); records, nodes and faces stay resident in the
+// 126 MB L2 for scenes up to a few million faces.
 
 #include <algorithm>
 #include <type_traits>
@@ -208,7 +209,7 @@ __global__ void __launch_bounds__(128, TL ? PT_WIDE_TL_BLOCKS : PT_WIDE_BLOCKS) 
                                                             int* err, unsigned long long* counter, uint32_t chunk, float size) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t warp = blockIdx.x * 4 + (threadIdx.x >> 5);
-    // this warp's rays: first its own chunk, then those that the counter hands out (base + chunk <= n + 2^12)
+    // this warp's rays: first its own chunk, then those that the counter hands out (base + take <= n + 2^13)
     uint32_t pool_next = warp * chunk < n ? warp * chunk : n, pool_end = n - pool_next < chunk ? n : pool_next + chunk;
     bool exhausted = false, loaded = false;  // loaded: the lane holds a ray whose hit is not yet stored
     uint32_t idx = 0;
@@ -263,15 +264,16 @@ __global__ void __launch_bounds__(128, TL ? PT_WIDE_TL_BLOCKS : PT_WIDE_BLOCKS) 
             }
             if (!exhausted && pool_next >= pool_end) {
                 unsigned long long base = (unsigned long long)gridDim.x * 4 * chunk;
+                const uint32_t take = TL ? chunk : wide_take(n - pool_end, gridDim.x * 4, chunk);
                 if (base < n) {
-                    if (lane == 0) base += atomicAdd(counter, (unsigned long long)chunk);
+                    if (lane == 0) base += atomicAdd(counter, (unsigned long long)take);
                     base = __shfl_sync(0xFFFFFFFFu, base, 0);
                 }
                 if (base >= n) {
                     exhausted = true;
                 } else {
                     pool_next = (uint32_t)base;
-                    pool_end = n - pool_next < chunk ? n : pool_next + chunk;
+                    pool_end = n - pool_next < take ? n : pool_next + take;
                 }
             }
             const uint32_t avail = pool_end - pool_next;

@@ -246,14 +246,15 @@ __global__ void __launch_bounds__(THREADS, 128 * PT_WIDE_BLOCKS / THREADS) wf_wi
                 loaded = false;
             }
             if (!exhausted && pool_next >= pool_end) {
+                const uint32_t take = wide_take(n - pool_end, gridDim.x * (THREADS / 32), chunk);
                 unsigned long long base = 0;
-                if (lane == 0) base = atomicAdd(fetch, (unsigned long long)chunk);
+                if (lane == 0) base = atomicAdd(fetch, (unsigned long long)take);
                 base = __shfl_sync(0xFFFFFFFFu, base, 0);
                 if (base >= n) {
                     exhausted = true;
                 } else {
                     pool_next = (uint32_t)base;
-                    pool_end = n - pool_next < chunk ? n : pool_next + chunk;
+                    pool_end = n - pool_next < take ? n : pool_next + take;
                 }
             }
             const uint32_t avail = pool_end - pool_next;
@@ -715,14 +716,15 @@ __global__ void __launch_bounds__(128, TL ? PT_WIDE_TL_BLOCKS : PT_WIDE_PATH_BLO
             // new paths for the idle lanes
             const uint32_t need = __ballot_sync(0xFFFFFFFFu, ended && !hit && todo == kIdle);
             if (need && !exhausted && pool_next >= pool_end) {
+                const uint32_t take = wide_take(count - pool_end, gridDim.x * 4, chunk);
                 unsigned long long base = 0;
-                if (lane == 0) base = atomicAdd(fetch, (unsigned long long)chunk);
+                if (lane == 0) base = atomicAdd(fetch, (unsigned long long)take);
                 base = __shfl_sync(0xFFFFFFFFu, base, 0);
                 if (base >= count) {
                     exhausted = true;
                 } else {
                     pool_next = (uint32_t)base;
-                    pool_end = base + chunk < count ? (uint32_t)base + chunk : count;
+                    pool_end = base + take < count ? (uint32_t)base + take : count;
                 }
             }
             const uint32_t avail = pool_end - pool_next;
@@ -1116,7 +1118,7 @@ cudaError_t launch_wide_paths(const WfItem* items, const WfSegment* segs, uint32
     if (e != cudaSuccess) return e;
     if (per_sm < 1) per_sm = 1;
     uint64_t grid = (uint64_t)sms * per_sm;
-    const uint64_t grid_needed = (((uint64_t)count + chunk - 1) / chunk * 32 + 127) / 128;
+    const uint64_t grid_needed = (((uint64_t)count + kWideFew - 1) / kWideFew * 32 + 127) / 128;
     if (grid > grid_needed) grid = grid_needed ? grid_needed : 1;
     e = cudaMemsetAsync(fetch, 0, sizeof(unsigned long long), s);
     if (e != cudaSuccess) return e;

@@ -33,6 +33,16 @@ def test_ray_counts_around_warps_chunks_and_grids(cuda_device, n):
     s.close()
 
 
+@pytest.mark.parametrize("chunk", [32, 64, 4096])
+@pytest.mark.parametrize("n", [378_881, 757_763, 1_515_521])
+def test_ray_counts_around_the_sizes_that_warps_take(cuda_device, n, chunk):
+    """On 148 SMs, twice, four and eight times the chunks of 64 that all warps hold at once, and one more."""
+    s = pb.Scene(W.small_scene(3)[0])
+    s.set_trace_tuning(16, chunk)
+    same_hits(s, np.resize(edge_case_rays(50_000, n), n))
+    s.close()
+
+
 @pytest.mark.parametrize("shared", [0, 8, 16, 24, 32])
 def test_shared_stack_depths(cuda_device, shared):
     s = pb.Scene(scene("boxes"))
