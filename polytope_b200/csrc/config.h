@@ -73,6 +73,19 @@
 #define PT_WIDE_LAST_LEAVES 2
 #endif
 
+// Resident blocks of 128 and leaf batch of the extend and shadow kernels (wf_wide_kernel).  Their rays come
+// from one wave and are alike, so more warps pay although the walk spills (72 registers, about 150 B).
+// Measured on a B200 (ms, four renders of depth 6; scenes of 500 k box faces / 20 k box faces / instanced
+// spheres, 33.5 M paths in one wave; the binary walk's kernel 61.0 / 65.0 / 16.1): 7 blocks and 12 59.5 /
+// 66.0 / 12.9, 6 and 12 60.5 / 67.0 / 13.1, 8 and 12 60.6 / 66.6 / 13.0, 5 and 16 65.3 / 71.0 / 13.6; with
+// waves of 4.2 M paths (binary 9.39 / 9.89 / 4.75) 8.68 / 9.30 / 2.93, 5 and 16 9.20 / 9.73 / 2.92.
+#ifndef PT_WIDE_WF_BLOCKS
+#define PT_WIDE_WF_BLOCKS 7
+#endif
+#ifndef PT_WIDE_WF_BATCH
+#define PT_WIDE_WF_BATCH 12
+#endif
+
 // The same for the persistent path kernel (wf_wide_path_kernel), with the lanes that must have a ray to
 // end or start, or a hit to shade, before those steps run.  Measured on a B200 (ms; 1920x1080x16 frame
 // of 3.9 M faces / 641x479x4 frame of 20 k box faces / 24 served requests), before the binary walk's
@@ -117,4 +130,11 @@
 // 8 % ahead (24 uneven renders, 24.5 against 26.3).
 #ifndef PT_WIDE_WAVE_PATHS
 #define PT_WIDE_WAVE_PATHS (1u << 17)
+#endif
+// Paths up to which a wave's extend and shadow kernels walk the records.  In longer waves all warps stay
+// busy with alike rays, and on box scenes the binary walk's 64 registers gain more than the records do: 256
+// uneven renders in waves of 33.5 M paths 1043 ms against 1073, four scenes of 20 k box faces 65.0 / 66.0
+// (of instanced spheres 16.1 / 12.9, which the path pipeline renders faster still); at 16.8 M 33.3 / 33.1.
+#ifndef PT_WIDE_WAVE_MOST
+#define PT_WIDE_WAVE_MOST (1u << 24)
 #endif

@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(256, kWfTraceMinBlocks) wf_trace_kernel(const 
 // PT_WIDE_BATCH lanes hold a leaf, then faces; ended lanes store their results and take queue entries
 // PT_WIDE_REFILL at a time.
 template <bool SHADOW, int THREADS>
-__global__ void __launch_bounds__(THREADS, 128 * PT_WIDE_BLOCKS / THREADS) wf_wide_kernel(const WfItem* __restrict__ items, WfState ws,
+__global__ void __launch_bounds__(THREADS, 128 * PT_WIDE_WF_BLOCKS / THREADS) wf_wide_kernel(const WfItem* __restrict__ items, WfState ws,
                                                        const uint32_t* __restrict__ queue, const uint32_t* count_ptr,
                                                        unsigned long long* fetch, uint32_t chunk,
                                                        unsigned long long* rays_traced) {
@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(THREADS, 128 * PT_WIDE_BLOCKS / THREADS) wf_wi
         const bool at_leaf = k.cur != kWideDone && (k.cur & kWideLeaf);
         const uint32_t leaves = __ballot_sync(0xFFFFFFFFu, at_leaf);
         const int live = __popc(~ended);
-        if (__popc(leaves) >= min(live, exhausted ? PT_WIDE_LAST_BATCH : PT_WIDE_BATCH)) {
+        if (__popc(leaves) >= min(live, exhausted ? PT_WIDE_LAST_BATCH : PT_WIDE_WF_BATCH)) {
 #pragma unroll 1
             for (int step = 0; step < (exhausted ? PT_WIDE_LAST_LEAVES : 1) && (k.cur & kWideLeaf) && k.cur != kWideDone; ++step) {
                 wide_faces(k, tris, [&]() { return (const uint4*)p->nodes; }, dir, []() { return 0u; });
@@ -1177,7 +1177,9 @@ cudaError_t trace_stage(const WfItem* items, const WfState& ws, const uint32_t* 
 // Camera rays of the wave's slots, then per bounce: extend, shade (queue the next rays and the
 // shadow rays), shadow; finally the clamped radiance of every slot.
 cudaError_t bounce_stages(const WfItem* d_items, const WfSegment* d_segments, const WfWave& w, const WfState& ws,
-                          const WfTuning& t, unsigned long long* rays_traced, cudaStream_t s) {
+                          const WfTuning& tuning, unsigned long long* rays_traced, cudaStream_t s) {
+    WfTuning t = tuning;
+    t.wide = t.wide && w.count <= PT_WIDE_WAVE_MOST;
     const uint32_t blocks = (w.count + 127) / 128;
     wf_init_kernel<<<blocks, 128, 0, s>>>(d_items, d_segments + w.seg_begin, w.seg_count, w.count, ws);
     cudaError_t e = cudaGetLastError();

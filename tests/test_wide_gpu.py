@@ -115,10 +115,12 @@ def test_batches_with_and_without_records(cuda_device, pipeline, threads):
 
 
 @pytest.mark.parametrize("threads", [64, 128, 256])
-@pytest.mark.parametrize("width, depth, spp, wave", [(512, 0, 1, 0), (513, 0, 1, 0), (512, 2, 3, 0), (513, 2, 3, 0), (515, 0, 3, 256 * 600)])
+@pytest.mark.parametrize("width, depth, spp, wave", [(512, 0, 1, 0), (513, 0, 1, 0), (512, 2, 3, 0), (513, 2, 3, 0), (515, 0, 3, 256 * 600),
+                                                       (512, 0, 128, 1 << 25), (512, 0, 129, 1 << 25)])
 def test_waves_around_the_whole_path_limit(cuda_device, threads, width, depth, spp, wave):
-    """Waves of up to 131,072 paths a bounce run as whole paths, larger ones bounce by bounce; the last
-    case has two of the one kind and one of the other in a batch."""
+    """Waves of up to 131,072 paths a bounce run as whole paths, larger ones bounce by bounce; the fifth
+    case has two of the one kind and one of the other in a batch.  Up to 2^24 paths those walk the records,
+    above the binary nodes."""
     s = pb.Scene(scene("boxes"), env=(51.0,) * 3)
     t = pb.default_tuning()
     t.pipeline, t.threads_per_block, t.wave_pixels = pb.PIPELINE_WAVEFRONT, threads, wave
