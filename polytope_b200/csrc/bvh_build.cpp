@@ -444,12 +444,15 @@ int validate_tree(const pt_bvh_node* nodes, uint32_t num_nodes, uint32_t num_lea
     std::vector<uint8_t> seen(num_nodes, 0);
     seen[0] = 1;
     uint32_t max_depth = 0, records = 0;
-    bool shared = false;  // a node with two parents: no record numbering by depth
+    bool numbered = true;  // not where a node has two parents (no numbering by depth), or none (never checked)
     if (wide_of) wide_of->assign(num_nodes, kNotWide);
     // Pre-order layout: every child index is larger than its parent's, so one forward sweep
     // visits parents first.
     for (uint32_t i = 0; i < num_nodes; ++i) {
-        if (!seen[i]) continue;
+        if (!seen[i]) {
+            numbered = false;
+            continue;
+        }
         const pt_bvh_node& n = nodes[i];
         max_depth = std::max(max_depth, depth[i]);
         if (wide_of && (i == 0 || (n.num_faces == 0 && (depth[i] & 1u) == 0))) (*wide_of)[i] = records++;
@@ -462,12 +465,12 @@ int validate_tree(const pt_bvh_node* nodes, uint32_t num_nodes, uint32_t num_lea
         const uint64_t lo = (uint64_t)i + 1, hi = (uint64_t)i + n.offset;
         if (n.offset < 2 || hi >= num_nodes || lo >= num_nodes)
             return fail(PT_EINVAL, "node " + std::to_string(i) + ": child index out of bounds");
-        shared = shared || seen[lo] || seen[hi];
+        numbered = numbered && !seen[lo] && !seen[hi];
         seen[lo] = seen[hi] = 1;
         depth[lo] = depth[hi] = depth[i] + 1;
     }
     if (max_depth_out) *max_depth_out = max_depth;
-    if (wide_of && (shared || num_nodes > (1u << 28))) {
+    if (wide_of && (!numbered || num_nodes > (1u << 28))) {
         wide_of->clear();
         records = 0;
     }

@@ -64,10 +64,11 @@ int build_bvh(const pt_mesh_desc* meshes, uint32_t num_meshes, const WorldMeshes
 int scene_trace(pt_scene* s, const pt_ray* rays, uint64_t n, pt_hit* hits, uint32_t* node_tests,
                 uint32_t* tri_tests, uint32_t mem_flags, void* stream);
 
-// Checks that every child / leaf range stays inside the arrays and computes the deepest level.
-// wide_of (optional) receives the number of the four-wide record (wide.cuh) that starts at each
-// node, kNotWide where none does, and num_wide their count: the root and the interior nodes at even
-// depth.  Empty when some node has two parents (a caller's own tree) or the indices do not fit.
+// Checks that the child and leaf ranges of every node that the root reaches stay inside the arrays and
+// computes the deepest level.  wide_of (optional) receives the number of the four-wide record
+// (wide.cuh) that starts at each node, kNotWide where none does, and num_wide their count: the root
+// and the interior nodes at even depth.  Empty when some node has two parents, or none (a caller's own
+// tree), or the indices do not fit: so all nodes of a numbered tree have been checked.
 constexpr uint32_t kNotWide = 0xFFFFFFFFu;
 constexpr float kWideSizeMin = 9.3132257e-10f, kWideSizeMax = 1.0737418e9f;  // 2^-30, 2^30: the trees wide.cuh is proved for
 int validate_tree(const pt_bvh_node* nodes, uint32_t num_nodes, uint32_t num_leaf_entries, uint32_t* max_depth,

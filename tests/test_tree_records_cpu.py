@@ -1,0 +1,27 @@
+"""Which trees get four-wide records (validate_tree's numbering), on the host: tests/cpp/tree_records_check.cpp
+linked against the library.  No device is used and no tree is uploaded."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+LIB = os.path.join(ROOT, "polytope_b200", "lib")
+
+pytestmark = pytest.mark.skipif(shutil.which("g++") is None, reason="needs g++")
+
+
+@pytest.fixture(scope="module")
+def harness(tmp_path_factory):
+    exe = tmp_path_factory.mktemp("records") / "tree_records_check"
+    subprocess.run(["g++", "-O1", "-std=c++17", "-Wall", "-I", os.path.join(ROOT, "polytope_b200", "csrc"),
+                    os.path.join(ROOT, "tests", "cpp", "tree_records_check.cpp"), "-o", str(exe),
+                    "-L", LIB, "-lpolytope_b200", "-Wl,-rpath," + LIB], check=True, capture_output=True, text=True)
+    return exe
+
+
+@pytest.mark.parametrize("case", ["numbered", "unreached"])
+def test_which_trees_are_numbered(harness, case):
+    p = subprocess.run([str(harness), case], capture_output=True, text=True, timeout=60)
+    assert p.returncode == 0 and p.stdout.strip() == "ok", p.stdout + p.stderr
