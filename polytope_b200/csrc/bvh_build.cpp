@@ -470,7 +470,7 @@ int validate_tree(const pt_bvh_node* nodes, uint32_t num_nodes, uint32_t num_lea
         depth[lo] = depth[hi] = depth[i] + 1;
     }
     if (max_depth_out) *max_depth_out = max_depth;
-    if (wide_of && (!numbered || num_nodes > (1u << 28))) {
+    if (wide_of && (!numbered || num_nodes > kWideNodesMost)) {
         wide_of->clear();
         records = 0;
     }

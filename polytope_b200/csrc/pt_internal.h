@@ -70,6 +70,9 @@ int scene_trace(pt_scene* s, const pt_ray* rays, uint64_t n, pt_hit* hits, uint3
 // and the interior nodes at even depth.  Empty when some node has two parents, or none (a caller's own
 // tree), or the indices do not fit: so all nodes of a numbered tree have been checked.
 constexpr uint32_t kNotWide = 0xFFFFFFFFu;
+// Nodes a tree with records has at most.  A slot's reference can name a node by 28 bits beneath four set
+// ones (a large leaf); all 28 set and the value below are the walk's own marks (kWideDone, kWideExit).
+constexpr uint32_t kWideNodesMost = (1u << 28) - 2;
 constexpr float kWideSizeMin = 9.3132257e-10f, kWideSizeMax = 1.0737418e9f;  // 2^-30, 2^30: the trees wide.cuh is proved for
 int validate_tree(const pt_bvh_node* nodes, uint32_t num_nodes, uint32_t num_leaf_entries, uint32_t* max_depth,
                   std::vector<uint32_t>* wide_of = nullptr, uint32_t* num_wide = nullptr);

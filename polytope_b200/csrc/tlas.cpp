@@ -234,7 +234,7 @@ int prepare_two_level_host(const pt_scene_desc* desc, HostScene& h) {
     uint32_t tdepth = 0, records = 0;
     rc = validate_tree(h.tlas.data(), (uint32_t)h.tlas.size(), (uint32_t)h.instances.size(), &tdepth, &h.top_wide_of, &records);
     if (rc) return fail(rc, std::string("top-level tree: ") + pt_last_error());
-    if (h.wide_of.size() == h.nodes.size() && !h.top_wide_of.empty() && h.nodes.size() < (1u << 28)) {
+    if (h.wide_of.size() == h.nodes.size() && !h.top_wide_of.empty() && h.nodes.size() <= kWideNodesMost) {
         for (uint32_t& r : h.wide_of) r = r == kNotWide ? r : r + records;  // the top level's records come first
         h.num_wide += records;
     } else {
