@@ -302,11 +302,7 @@ __global__ void __launch_bounds__(128, TL ? PT_WIDE_TL_BLOCKS : PT_WIDE_BLOCKS) 
                 if (crosses) {
                     const float4 r0 = rays[2 * (size_t)idx], r1 = rays[2 * (size_t)idx + 1];
                     F3 o = f3(r0.x, r0.y, r0.z), d = f3(r1.x, r1.y, r1.z);
-                    if (k.cur == kWideExit) {
-                        inside = false;
-                        wide_pop(k);
-                    }
-                    const bool enters = (k.cur & kWideLeaf) && k.cur != kWideDone;
+                    const bool enters = wide_cross(k, inside);
                     if (k.cur != kWideDone) {  // into an instance, or back to a top-level record
                         const uint32_t ii = k.cur & kWideIndex;
                         uint4 wi = make_uint4(0u, __float_as_uint(size), 0u, 0u);

@@ -803,12 +803,9 @@ __global__ void __launch_bounds__(128, TL ? PT_WIDE_TL_BLOCKS : PT_WIDE_PATH_BLO
             if (crosses) {
                 o = cold.f3at(kPo);
                 d = cold.f3at((state & kRayMask) == kOnShadow ? kPw : kPd);
-                if (k.cur == kWideExit) {
-                    inside = false;
-                    wide_pop(k);
-                    if (!(k.cur & kWideLeaf)) setup = kLeave;
-                }
-                if ((k.cur & kWideLeaf) && k.cur != kWideDone) {
+                const bool leaves_one = k.cur == kWideExit, enters = wide_cross(k, inside);
+                if (leaves_one && !(k.cur & kWideLeaf)) setup = kLeave;
+                if (enters) {
                     cold.set(kPinst, k.cur & kWideIndex);
                     cold.set(kPentry, k.min_t);
                     sure = false;

@@ -36,6 +36,7 @@ namespace pt {
 constexpr uint32_t kWideLeaf = 0x80000000u;   // slot is a leaf: faces (ref >> 28) & 7 from ref & kWideIndex
 constexpr uint32_t kWideIndex = 0x0FFFFFFFu;
 constexpr uint32_t kWideBig = 7u;             // leaf of more than 6 faces: the index names its binary node
+constexpr uint32_t kWideEmpty = kWideLeaf;    // empty slot: a leaf without faces (visited or entered by no walk)
 constexpr uint32_t kWideDone = 0xFFFFFFFFu;   // no slot's reference: WideWalkT::cur at the end of a walk
 constexpr int kWideStack = 100;               // 1 + 3 entries a level, 32 levels of two binary ones each
 
@@ -98,7 +99,7 @@ PT_HD bool wide_make(const uint4* nodes, const uint32_t* wide_of, uint32_t ni, f
     bool full[4] = {false, false, false, false}, ok = true;
     uint32_t axis[3] = {0, 0, 0};
     uint4 pb;
-    for (int s = 0; s < 4; ++s) w.ref[s] = kWideLeaf;  // empty: a leaf without faces
+    for (int s = 0; s < 4; ++s) w.ref[s] = kWideEmpty;
     wide_box(nodes, ni, plo, phi, pb);
     auto inside = [&](const float* l, const float* h, const float* ol, const float* oh) {
         for (int k = 0; k < 3; ++k) ok = ok && ol[k] <= l[k] && l[k] <= h[k] && h[k] <= oh[k];
@@ -143,7 +144,9 @@ PT_HD bool wide_make(const uint4* nodes, const uint32_t* wide_of, uint32_t ni, f
         for (int s = 0; s < 4; ++s) {
             // a 32nd of a step outwards on top of the rounding: it covers the rounding errors of these
             // differences (at most 2^-16 of a step) and, in wide_visit, those that go with the step
-            uint32_t a = 255u, b = 0u;  // empty: low plane beyond the high one on every axis
+            // empty: low plane beyond the high one on every axis, which stops all rays but those from afar,
+            // whose slack (wide_visit) is wider than the record; they pass over the reference (kWideEmpty)
+            uint32_t a = 255u, b = 0u;
             if (full[s]) {
                 const float x = floorf(fsub(fsub(fmul(lo[s][k], inv), first), 0.03125f));
                 const float y = ceilf(fadd(fsub(fmul(hi[s][k], inv), first), 0.03125f));
@@ -481,6 +484,18 @@ PT_HD void wide_to_object(const DeviceInstance* inst, V& o, V& d) {
     const V wo = o, wd = d;
     to_object(m, wo.x, wo.y, wo.z, 1.0f, o.x, o.y, o.z);
     to_object(m, wd.x, wd.y, wd.z, 0.0f, d.x, d.y, d.z);
+}
+
+// A lane at an exit marker or a top-level leaf: leaves its instance (inside), if it is in one, and passes over
+// empty slots.  Returns whether k.cur is then an instance to enter (else a top-level record, or kWideDone).
+template <int CAP, int SH>
+PT_HD bool wide_cross(WideWalkT<CAP, SH>& k, bool& inside) {
+    if (k.cur == kWideExit) {
+        inside = false;
+        wide_pop(k);
+    }
+    while (k.cur == kWideEmpty) wide_pop(k);
+    return (k.cur & kWideLeaf) && k.cur != kWideDone;
 }
 
 // Enters the instance whose tree starts at record root, with its object ray in k.r.  False when that ray is
