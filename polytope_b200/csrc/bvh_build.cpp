@@ -444,8 +444,14 @@ int validate_tree(const pt_bvh_node* nodes, uint32_t num_nodes, uint32_t num_lea
     std::vector<uint8_t> seen(num_nodes, 0);
     seen[0] = 1;
     uint32_t max_depth = 0, records = 0;
-    bool numbered = true;  // not where a node has two parents (no numbering by depth), or none (never checked)
-    if (wide_of) wide_of->assign(num_nodes, kNotWide);
+    // not where a node has two parents (no numbering by depth), or none (never checked), nor where two leaves
+    // share a face (whose record names one leaf)
+    bool numbered = true;
+    std::vector<uint8_t> taken;  // faces of the leaves so far
+    if (wide_of) {
+        wide_of->assign(num_nodes, kNotWide);
+        taken.assign(num_leaf_entries, 0);
+    }
     // Pre-order layout: every child index is larger than its parent's, so one forward sweep
     // visits parents first.
     for (uint32_t i = 0; i < num_nodes; ++i) {
@@ -459,6 +465,11 @@ int validate_tree(const pt_bvh_node* nodes, uint32_t num_nodes, uint32_t num_lea
         if (n.num_faces > 0) {
             if ((uint64_t)n.offset + n.num_faces > num_leaf_entries)
                 return fail(PT_EINVAL, "leaf " + std::to_string(i) + " face range out of bounds");
+            if (wide_of) {
+                uint8_t *first = taken.data() + n.offset, *last = first + n.num_faces;
+                numbered = numbered && std::find(first, last, (uint8_t)1) == last;
+                std::fill(first, last, (uint8_t)1);
+            }
             continue;
         }
         if (n.axis > 2) return fail(PT_EINVAL, "node " + std::to_string(i) + ": bad split axis");

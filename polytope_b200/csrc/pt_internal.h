@@ -67,8 +67,9 @@ int scene_trace(pt_scene* s, const pt_ray* rays, uint64_t n, pt_hit* hits, uint3
 // Checks that the child and leaf ranges of every node that the root reaches stay inside the arrays and
 // computes the deepest level.  wide_of (optional) receives the number of the four-wide record
 // (wide.cuh) that starts at each node, kNotWide where none does, and num_wide their count: the root
-// and the interior nodes at even depth.  Empty when some node has two parents, or none (a caller's own
-// tree), or the indices do not fit: so all nodes of a numbered tree have been checked.
+// and the interior nodes at even depth.  Empty when some node has two parents, or none, or two leaves
+// share a face (a caller's own tree), or the indices do not fit: so all nodes of a numbered tree have
+// been checked, and each face record has room for the one leaf that holds it.
 constexpr uint32_t kNotWide = 0xFFFFFFFFu;
 // Nodes a tree with records has at most.  A slot's reference can name a node by 28 bits beneath four set
 // ones (a large leaf); all 28 set and the value below are the walk's own marks (kWideDone, kWideExit).

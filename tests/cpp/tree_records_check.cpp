@@ -63,10 +63,24 @@ static void unreached() {
     }
 }
 
+// Two leaves over the same faces, the whole range or a part of it, in either order: no records, and the
+// tree is accepted as one without them is.  Leaves that meet without sharing a face are numbered.
+static void shared_faces() {
+    struct { uint32_t a, na, b, nb; bool shares; } const cases[] = {
+        {0, 2, 0, 2, true}, {0, 3, 2, 2, true}, {2, 2, 0, 3, true}, {0, 4, 1, 2, true}, {1, 2, 0, 4, true},
+        {0, 2, 2, 2, false}, {2, 2, 0, 2, false}, {0, 1, 3, 1, false}};
+    for (const auto& c : cases) {
+        const Result r({inner(2), leaf(c.a, (uint16_t)c.na), leaf(c.b, (uint16_t)c.nb)}, 4);
+        CHECK(r.rc == PT_OK && r.depth == 1);
+        CHECK(c.shares ? r.none() : r.records == 1 && r.wide_of.size() == 3);
+    }
+}
+
 int main(int argc, char** argv) {
     const char* name = argc == 2 ? argv[1] : "";
     if (!std::strcmp(name, "numbered")) numbered();
     else if (!std::strcmp(name, "unreached")) unreached();
+    else if (!std::strcmp(name, "shared_faces")) shared_faces();
     else return 2;
     if (failures == 0) std::puts("ok");
     return failures ? 1 : 0;

@@ -24,7 +24,7 @@ def harness(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("case", ["numbered", "unreached"])
+@pytest.mark.parametrize("case", ["numbered", "unreached", "shared_faces"])
 def test_which_trees_are_numbered(harness, case):
     p = subprocess.run([str(harness), case], capture_output=True, text=True, timeout=60)
     assert p.returncode == 0 and p.stdout.strip() == "ok", p.stdout + p.stderr
