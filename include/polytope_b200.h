@@ -143,7 +143,7 @@ int pt_scene_create(const pt_scene_desc *desc, pt_scene **out);
 int pt_scene_create_two_level(const pt_scene_desc *desc, pt_scene **out);
 
 /* What pt_scene_create_two_level would build from `desc`, computed on the host alone (no device
- * needed): counts and the device bytes the scene would hold. */
+ * needed): counts and the device bytes of the scene's arrays (pt_scene_info.device_bytes). */
 typedef struct pt_two_level_info {
     uint32_t num_instances, num_geometries;
     uint32_t blas_nodes, blas_faces;    /* bottom-level trees and faces, all geometries   */
@@ -161,10 +161,15 @@ typedef struct pt_scene_info {
     uint32_t num_prims;
     uint32_t num_meshes;
     uint32_t max_depth;            /* deepest node level (root = 0)                           */
-    uint64_t device_bytes;         /* nodes, faces and the other arrays of the description (the
-                                    * four-wide records, about a quarter more, are not counted)*/
+    uint64_t device_bytes;         /* nodes, faces and the other arrays of the description;
+                                    * pt_scene_device_memory counts all that the handle holds  */
 } pt_scene_info;
 int pt_scene_get_info(const pt_scene *scene, pt_scene_info *info);
+
+/* Device memory that the handle holds now: the arrays of pt_scene_info.device_bytes, the four-wide
+ * records made from them (about a quarter more; none for a tree that keeps the binary walk), and
+ * from the first pt_trace with host arrays on its staging buffers. */
+int pt_scene_device_memory(pt_scene *scene, uint64_t *bytes);
 
 /* ---- ray queries (Scene::intersect) ------------------------------------------------------ */
 

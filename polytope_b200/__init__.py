@@ -165,6 +165,7 @@ def _load() -> C.CDLL:
         "pt_scene_create_two_level": (i, [C.POINTER(SceneDesc), C.POINTER(_vp)]),
         "pt_scene_destroy": (i, [_vp]),
         "pt_scene_get_info": (i, [_vp, C.POINTER(SceneInfo)]),
+        "pt_scene_device_memory": (i, [_vp, C.POINTER(C.c_uint64)]),
         "pt_trace": (i, [_vp, _vp, u64, _vp, u32, _vp]),
         "pt_trace_counted": (i, [_vp, _vp, u64, _vp, _vp, _vp, u32, _vp]),
         "pt_render": (i, [_vp, C.POINTER(RenderDesc), _vp, _vp, u32, _vp]),
@@ -390,6 +391,12 @@ class Scene:
         inf = SceneInfo()
         check(lib.pt_scene_get_info(self.handle, C.byref(inf)))
         return inf
+
+    def device_memory(self) -> int:
+        """Device memory that the handle holds now (pt_scene_device_memory)."""
+        n = C.c_uint64()
+        check(lib.pt_scene_device_memory(self.handle, C.byref(n)))
+        return n.value
 
     def intersect(self, rays, hits=None, device: bool = False, stream: int = 0, counts: bool = False):
         """Scene::intersect for a batch: numpy (host) arrays, or torch CUDA tensors with device=True

@@ -133,17 +133,17 @@ bool is_pinned(const void* p) {
 // 1 M-ray chunks 1436 Mrays/s, 512 K 1413, 2 M 1339 (longer fill and drain), 256 K 1030.
 constexpr size_t kChunkRays = size_t(1) << 20;
 constexpr int kSlots = 4;  // chunks in flight: one being copied in, one or two in kernels, one copied out
+constexpr size_t kStagingIn = kSlots * kChunkRays * sizeof(pt_ray), kStagingOut = kSlots * kChunkRays * sizeof(pt_hit);
 
 int ensure_staging(pt_scene* s) {
     if (s->staging_rays) return PT_OK;
     for (void*& st : s->streams) PT_CUDA(cudaStreamCreateWithFlags((cudaStream_t*)&st, cudaStreamNonBlocking));
     for (int i = 0; i < 3 * kSlots + 1; ++i)
         PT_CUDA(cudaEventCreateWithFlags((cudaEvent_t*)&s->events[i], cudaEventDisableTiming));
-    const size_t in_b = kSlots * kChunkRays * sizeof(pt_ray), out_b = kSlots * kChunkRays * sizeof(pt_hit);
-    if (cudaMalloc(&s->dev_in, in_b) != cudaSuccess || cudaMalloc(&s->dev_out, out_b) != cudaSuccess ||
+    if (cudaMalloc(&s->dev_in, kStagingIn) != cudaSuccess || cudaMalloc(&s->dev_out, kStagingOut) != cudaSuccess ||
         cudaMalloc(&s->trace_err, sizeof(int)) != cudaSuccess)
         return fail(PT_ENOMEM, "cudaMalloc staging buffers");
-    if (cudaMallocHost(&s->pin_in, in_b) != cudaSuccess || cudaMallocHost(&s->pin_out, out_b) != cudaSuccess)
+    if (cudaMallocHost(&s->pin_in, kStagingIn) != cudaSuccess || cudaMallocHost(&s->pin_out, kStagingOut) != cudaSuccess)
         return fail(PT_ENOMEM, "cudaMallocHost staging buffers");
     s->staging_rays = kChunkRays;
     return PT_OK;
@@ -568,6 +568,7 @@ int create_from_host(const pt_scene_desc* desc, HostScene& h, pt_scene** out) {
         free_scene(s.release());
         return fail(PT_ENOMEM, std::string("cudaMalloc scene memory: ") + cudaGetErrorString(e));
     }
+    s->memory_bytes = total + wide;
     char* at = (char*)s->memory;
     s->err_flag = at;
     s->ray_counters = at + 256;
@@ -651,6 +652,13 @@ int pt_scene_get_info(const pt_scene* s, pt_scene_info* info) {
     info->num_meshes = s->num_meshes;
     info->max_depth = s->max_depth;
     info->device_bytes = s->device_bytes;
+    return PT_OK;
+}
+
+int pt_scene_device_memory(pt_scene* s, uint64_t* bytes) {
+    if (!s || !bytes) return fail(PT_EINVAL, "scene or bytes is NULL");
+    std::lock_guard<std::mutex> lock(s->staging_mu);
+    *bytes = s->memory_bytes + (s->staging_rays ? kStagingIn + kStagingOut + sizeof(int) : 0);
     return PT_OK;
 }
 

@@ -152,6 +152,7 @@ struct SceneDev {
 struct pt_scene {
     pt::SceneDev dev;
     void* memory = nullptr;  // the allocation that holds all of dev, the error flag and the ray counters
+    size_t memory_bytes = 0;
     uint32_t num_nodes = 0;
     uint32_t num_prims = 0;
     uint32_t num_meshes = 0;
