@@ -803,9 +803,9 @@ __global__ void __launch_bounds__(128, TL ? PT_WIDE_TL_BLOCKS : PT_WIDE_PATH_BLO
             if (crosses) {
                 o = cold.f3at(kPo);
                 d = cold.f3at((state & kRayMask) == kOnShadow ? kPw : kPd);
-                const bool leaves_one = k.cur == kWideExit, enters = wide_cross(k, inside);
-                if (leaves_one && !(k.cur & kWideLeaf)) setup = kLeave;
-                if (enters) {
+                if (!wide_cross(k, inside)) {
+                    if (k.cur != kWideDone) setup = kLeave;
+                } else {
                     cold.set(kPinst, k.cur & kWideIndex);
                     cold.set(kPentry, k.min_t);
                     sure = false;

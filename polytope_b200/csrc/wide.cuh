@@ -486,16 +486,16 @@ PT_HD void wide_to_object(const DeviceInstance* inst, V& o, V& d) {
     to_object(m, wd.x, wd.y, wd.z, 0.0f, d.x, d.y, d.z);
 }
 
-// A lane at an exit marker or a top-level leaf: leaves its instance (inside), if it is in one, and passes over
-// empty slots.  Returns whether k.cur is then an instance to enter (else a top-level record, or kWideDone).
+// A lane at an exit marker or a top-level leaf: leaves its instance (inside), if it is in one, or passes over
+// an empty slot.  Returns whether k.cur is then an instance to enter; else it is a top-level record, another
+// empty slot (for the next crossing), or kWideDone.
 template <int CAP, int SH>
 PT_HD bool wide_cross(WideWalkT<CAP, SH>& k, bool& inside) {
-    if (k.cur == kWideExit) {
+    if (k.cur == kWideExit || k.cur == kWideEmpty) {
         inside = false;
         wide_pop(k);
     }
-    while (k.cur == kWideEmpty) wide_pop(k);
-    return (k.cur & kWideLeaf) && k.cur != kWideDone;
+    return (k.cur & kWideLeaf) && k.cur != kWideEmpty && k.cur != kWideDone;
 }
 
 // Enters the instance whose tree starts at record root, with its object ray in k.r.  False when that ray is
