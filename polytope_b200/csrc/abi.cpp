@@ -51,10 +51,20 @@ float largest_coordinate(const pt_bvh_node& root) {
     return m;
 }
 
-// The four-wide records of the scene's trees (wide.cuh), made on the device from the uploaded nodes.  A
-// tree with a box outside its parent's (only a caller's own tree can have one) or of extreme size gets
-// none and keeps the binary walk, as does one whose records do not fit in memory.  `base` holds
-// wide_bytes(h): the instance table, the records, then the numbering and a flag.
+// The four-wide records of the scene's trees (wide.cuh), made on the device from the uploaded nodes.  Trees of
+// extreme size (wide_sizes_fit) get none and keep the binary walk, as do those with a box outside its
+// parent's (only a caller's own tree can have one) and those whose records do not fit in memory.  `base`
+// holds wide_bytes(h): the instance table, the records, then the numbering and a flag.
+bool wide_sizes_fit(const HostScene& h) {
+    auto fits = [](const pt_bvh_node& root) {
+        const float size = largest_coordinate(root);
+        return size >= kWideSizeMin && size <= kWideSizeMax;
+    };
+    if (!h.two_level) return fits(h.nodes[0]);
+    bool all = fits(h.tlas[0]);
+    for (const HostScene::Geometry& g : h.geometries) all = all && fits(h.nodes[g.node_base]);
+    return all;
+}
 size_t wide_table_bytes(const HostScene& h) { return up256(sizeof(WideInstance) * h.instances.size()); }
 size_t wide_bytes(const HostScene& h) {
     return wide_table_bytes(h) + 64 * (size_t)h.num_wide + 4 * (h.wide_of.size() + h.top_wide_of.size() + 1);
@@ -82,24 +92,19 @@ int make_wide(pt_scene* s, const HostScene& h, char* base) {
     } else {
         trees.push_back({s->dev.nodes, number, (uint32_t)n, 0, largest_coordinate(h.nodes[0]), true});
     }
-    bool fits = true;
-    for (const Tree& t : trees) fits = fits && t.size >= kWideSizeMin && t.size <= kWideSizeMax;
     uint32_t outside = 0;
-    cudaError_t e = cudaSuccess;
-    if (fits) {
-        e = cudaMemcpy(number, h.wide_of.data(), 4 * n, cudaMemcpyHostToDevice);
-        if (e == cudaSuccess && nt) e = cudaMemcpy(number + n, h.top_wide_of.data(), 4 * nt, cudaMemcpyHostToDevice);
-        if (e == cudaSuccess && !table.empty())
-            e = cudaMemcpy(records - sizeof(WideInstance) * table.size(), table.data(), sizeof(WideInstance) * table.size(), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMemset(number + n + nt, 0, 4);
-        for (const Tree& t : trees)
-            if (e == cudaSuccess)
-                e = launch_wide_make(t.nodes, t.wide_of, t.num_nodes, t.size, t.face_base, records, t.faces ? s->dev.tris : nullptr,
-                                     number + n + nt, nullptr);
-        if (e == cudaSuccess) e = cudaMemcpy(&outside, number + n + nt, 4, cudaMemcpyDeviceToHost);
-        if (e != cudaSuccess) return cuda_fail(e, "four-wide records");
-    }
-    if (!fits || outside) return PT_OK;
+    cudaError_t e = cudaMemcpy(number, h.wide_of.data(), 4 * n, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && nt) e = cudaMemcpy(number + n, h.top_wide_of.data(), 4 * nt, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && !table.empty())
+        e = cudaMemcpy(records - sizeof(WideInstance) * table.size(), table.data(), sizeof(WideInstance) * table.size(), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemset(number + n + nt, 0, 4);
+    for (const Tree& t : trees)
+        if (e == cudaSuccess)
+            e = launch_wide_make(t.nodes, t.wide_of, t.num_nodes, t.size, t.face_base, records, t.faces ? s->dev.tris : nullptr,
+                                 number + n + nt, nullptr);
+    if (e == cudaSuccess) e = cudaMemcpy(&outside, number + n + nt, 4, cudaMemcpyDeviceToHost);
+    if (e != cudaSuccess) return cuda_fail(e, "four-wide records");
+    if (outside) return PT_OK;
     s->dev.wide = records;
     s->wide_size = trees[0].size;
     return PT_OK;
@@ -554,7 +559,7 @@ int create_from_host(const pt_scene_desc* desc, HostScene& h, pt_scene** out) {
                           part(&s->dev.tlas_nodes, h.tlas)};
     size_t total = 256 + up256(8 * PT_RAY_COUNTERS);  // the error flag, the ray counters
     for (const Part& p : parts) total += up256(p.bytes);
-    size_t wide = h.wide_of.empty() || s->nan_boxes ? 0 : wide_bytes(h);
+    size_t wide = h.wide_of.empty() || s->nan_boxes || !wide_sizes_fit(h) ? 0 : wide_bytes(h);
     DeviceGuard g(s->device);
     cudaError_t e = cudaMalloc(&s->memory, total + wide);
     if (e != cudaSuccess && wide) {
@@ -586,6 +591,28 @@ int create_from_host(const pt_scene_desc* desc, HostScene& h, pt_scene** out) {
         return cuda_fail(e, "scene upload");
     }
     if (wide && (rc = make_wide(s.get(), h, at))) { free_scene(s.release()); return rc; }
+    if (wide && !s->dev.wide) {  // no records after all: their room goes back
+        void* less = nullptr;
+        e = cudaMalloc(&less, total);
+        if (e == cudaSuccess) {
+            char *from = (char*)s->memory, *to = (char*)less;
+            e = cudaMemcpy(to, from, total, cudaMemcpyDeviceToDevice);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+            for (const Part& p : parts)
+                if (p.bytes) *p.dst = to + ((char*)*p.dst - from);
+            s->err_flag = to;
+            s->ray_counters = to + 256;
+            s->memory = to;
+            s->memory_bytes = total;
+            cudaFree(from);
+            if (e != cudaSuccess) {
+                free_scene(s.release());
+                return cuda_fail(e, "scene upload");
+            }
+        } else {
+            cudaGetLastError();
+        }
+    }
     *out = s.release();
     return PT_OK;
 }
