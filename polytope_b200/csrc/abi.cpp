@@ -5,14 +5,15 @@
 #include <cstdio>
 #include <cstring>
 #include <memory>
+#include <new>
 #include <string>
-#include <system_error>
 #include <thread>
 #include <vector>
 
 #include <cuda_runtime.h>
 
 #include "exact_math.h"
+#include "host_workers.h"
 #include "launch.h"
 #include "pt_internal.h"
 
@@ -168,9 +169,6 @@ int fail(int code, const std::string& msg) {
 // (one thread: 5.9 ms for 1 M rays on a host of 16 threads, of which the kernel takes 0.3), so it is what
 // runs in parallel, and one worker's copies overlap another's transfers and kernel: 2.0 ms with eight;
 // 16 M rays 76.9 -> 24 ms; 70 k rays 0.53 -> 0.49.
-constexpr int kWorkers = 8;
-constexpr uint64_t kPageableRays = 1 << 16;  // below, the threads cost more than they bring
-
 static int trace_pageable(pt_scene* s, const TraceArgs& common, const pt_ray* rays, uint64_t n, pt_hit* hits, bool pin_rays,
                           bool pin_hits, cudaEvent_t dep) {
     const int workers = (int)std::min<uint64_t>({(uint64_t)kWorkers, std::max(2u, std::thread::hardware_concurrency()) / 2, n >> 15});
@@ -211,27 +209,23 @@ static int trace_pageable(pt_scene* s, const TraceArgs& common, const pt_ray* ra
             }
             return PT_OK;
         };
-        const int r = run();
+        int r = PT_ENOMEM;
+        try {
+            r = run();
+        } catch (const std::bad_alloc&) {  // a message found no memory
+            g_last_error = "no host memory";
+        }
         if (r != PT_OK) {
-            std::lock_guard<std::mutex> lock(mu);
+            std::unique_lock<std::mutex> lock(mu);
             if (!failed.exchange(true)) {
                 rc = r;
-                message = g_last_error;
+                message.swap(g_last_error);
             }
+            lock.unlock();
             cudaStreamSynchronize((cudaStream_t)s->streams[w]);  // nothing of this call still uses the arrays
         }
     };
-    std::vector<std::thread> pool;
-    pool.reserve(workers);
-    for (int w = 1; w < workers; ++w) {
-        try {
-            pool.emplace_back(work, w);
-        } catch (const std::system_error&) {
-            break;  // no more threads: fewer workers
-        }
-    }
-    work(0);
-    for (std::thread& t : pool) t.join();
+    run_workers(workers, work);
     return rc == PT_OK ? PT_OK : fail(rc, message);
 }
 
