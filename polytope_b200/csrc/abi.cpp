@@ -170,8 +170,7 @@ int fail(int code, const std::string& msg) {
 // runs in parallel, and one worker's copies overlap another's transfers and kernel: 2.0 ms with eight;
 // 16 M rays 76.9 -> 24 ms; 70 k rays 0.53 -> 0.49.
 static int trace_pageable(pt_scene* s, const TraceArgs& common, const pt_ray* rays, uint64_t n, pt_hit* hits, bool pin_rays,
-                          bool pin_hits, cudaEvent_t dep) {
-    const int workers = (int)std::min<uint64_t>({(uint64_t)kWorkers, std::max(2u, std::thread::hardware_concurrency()) / 2, n >> 15});
+                          bool pin_hits, cudaEvent_t dep, int workers) {
     constexpr uint64_t slot_rays = kSlots * kChunkRays / kWorkers;
     // at least two chunks a worker, so that its second copy-in follows the first's results closely
     const uint64_t chunk = std::min(slot_rays, (n + 2 * workers - 1) / (2 * workers)), chunks = (n + chunk - 1) / chunk;
@@ -281,8 +280,9 @@ int scene_trace(pt_scene* s, const pt_ray* rays, uint64_t n, pt_hit* hits, uint3
     PT_CUDA(cudaMemsetAsync(s->trace_err, 0, sizeof(int), h2d));  // before every copy-in, so before every kernel
     const bool pin_rays = is_pinned(rays), pin_hits = is_pinned(hits);
     const bool counted = node_tests || tri_tests;
-    if (!counted && !(pin_rays && pin_hits) && n >= kPageableRays) {
-        rc = trace_pageable(s, a, rays, n, hits, pin_rays, pin_hits, dep);
+    const int workers = counted || (pin_rays && pin_hits) ? 1 : pageable_workers(n, std::thread::hardware_concurrency(), one_processor());
+    if (workers > 1) {
+        rc = trace_pageable(s, a, rays, n, hits, pin_rays, pin_hits, dep, workers);
         if (rc) return rc;
         int err = 0;
         PT_CUDA(cudaMemcpy(&err, s->trace_err, sizeof(int), cudaMemcpyDeviceToHost));

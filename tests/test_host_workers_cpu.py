@@ -1,5 +1,5 @@
 """The host threads of pt_trace's pageable arrays (polytope_b200/csrc/host_workers.h): all work is done with
-however many threads the system gives, also when it has no memory for one."""
+however many threads the system gives, also when it has no memory for one, and one processor gets none."""
 import os
 import shutil
 import subprocess
@@ -11,7 +11,7 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 pytestmark = pytest.mark.skipif(shutil.which("g++") is None, reason="needs g++")
 
 
-@pytest.mark.parametrize("case", ["threads"])
+@pytest.mark.parametrize("case", ["threads", "counts"])
 def test_host_workers(tmp_path, case):
     exe = tmp_path / "host_workers_check"
     subprocess.run(["g++", "-O1", "-std=c++17", "-Wall", "-pthread", "-I", os.path.join(ROOT, "polytope_b200", "csrc"),
