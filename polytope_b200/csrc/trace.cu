@@ -218,7 +218,9 @@ __global__ void __launch_bounds__(128, TL ? PT_WIDE_TL_BLOCKS : PT_WIDE_BLOCKS) 
     __shared__ float sentry[TL ? 128 : 1];
     bool sure = true;                         // a face was accepted in it: its box has passed
     bool inside = !TL;                        // the walk is in an instance (or the scene is flattened)
-    WideWalkT<kWideStack, SH> k;
+    WideSpill<SH, TL> spill;
+    WideWalkT<kWideStack, SH, true> k;
+    k.stack.spill = spill.pairs;
     k.stack.base = sstack + threadIdx.x;
     k.stack.stride = 128;
     k.cur = kWideDone;
@@ -242,15 +244,16 @@ __global__ void __launch_bounds__(128, TL ? PT_WIDE_TL_BLOCKS : PT_WIDE_BLOCKS) 
                 uint4 h;
                 if (k.binary) {
                     const float4 r0 = rays[2 * (size_t)idx], r1 = rays[2 * (size_t)idx + 1];
-                    const BinaryRay ray{r0.x, r0.y, r0.z, r1.x, r1.y, r1.z, r0.w, k.any};
-                    BinaryHit b;
+                    auto& rest = spill.rest;
+                    rest.ray = BinaryRay{r0.x, r0.y, r0.z, r1.x, r1.y, r1.z, r0.w, k.any};
                     if constexpr (TL) {
                         const TwoLevelView view{nodes, tris, num_nodes, top, num_top, inst, false};
                         uint32_t hit_inst;
-                        ok = wide_two_level_walk(&view, &ray, &b, &hit_inst);
+                        ok = wide_two_level_walk(&view, &rest.ray, &rest.hit, &hit_inst, rest.stack);
                     } else {
-                        ok = wide_binary_walk(nodes, tris, num_nodes, &ray, &b);
+                        ok = wide_binary_walk(nodes, tris, num_nodes, &rest.ray, &rest.hit, rest.stack);
                     }
+                    const BinaryHit b = rest.hit;
                     h = make_uint4(b.prim, __float_as_uint(b.t), __float_as_uint(b.u), __float_as_uint(b.v));
                 } else {
                     h = make_uint4(k.prim, __float_as_uint(k.min_t), __float_as_uint(k.u), __float_as_uint(k.v));

@@ -122,9 +122,10 @@ PT_COLD int blas_walk_general(const TwoLevelView* v, const RayState* r, int mode
     return blas_walk<false, CAP, false, true>(*v, *r, mode, root, fbase, pbase, ii, any, stack, *min_t, *out);
 }
 
-template <bool COUNT, int CAP = kStackCap, bool SPLIT = false>
-PT_HD TwoLevelHit traverse_two_level(const TwoLevelView& v, float ox, float oy, float oz, float dx, float dy, float dz,
-                                     float tmax, bool any) {
+// tstack, stack: room for kTopStackCap and CAP entries.
+template <bool COUNT, int CAP, bool SPLIT>
+PT_HD TwoLevelHit traverse_two_level_on(uint32_t* tstack, uint32_t* stack, const TwoLevelView& v, float ox, float oy, float oz,
+                                        float dx, float dy, float dz, float tmax, bool any) {
     TwoLevelHit out;
     TraceResult& res = out.r;
     res.prim = kPrimNone;
@@ -138,10 +139,8 @@ PT_HD TwoLevelHit traverse_two_level(const TwoLevelView& v, float ox, float oy, 
     ray_setup(wr, ox, oy, oz, dx, dy, dz);
     const int wmode = box_mode_for(wr, tmax, v.exact_tree);
     float min_t = tmax;
-    uint32_t tstack[kTopStackCap];
     int tsp = 0;
     tstack[tsp++] = 0;
-    uint32_t stack[CAP];
     while (tsp > 0) {
         const uint32_t ti = tstack[--tsp];
         if (ti >= v.top_nodes) { res.overflow = true; return out; }
@@ -190,6 +189,13 @@ PT_HD TwoLevelHit traverse_two_level(const TwoLevelView& v, float ox, float oy, 
         }
     }
     return out;
+}
+
+template <bool COUNT, int CAP = kStackCap, bool SPLIT = false>
+PT_HD TwoLevelHit traverse_two_level(const TwoLevelView& v, float ox, float oy, float oz, float dx, float dy, float dz,
+                                     float tmax, bool any) {
+    uint32_t tstack[kTopStackCap], stack[CAP];
+    return traverse_two_level_on<COUNT, CAP, SPLIT>(tstack, stack, v, ox, oy, oz, dx, dy, dz, tmax, any);
 }
 
 }  // namespace pt

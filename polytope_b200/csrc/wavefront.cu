@@ -206,7 +206,9 @@ __global__ void __launch_bounds__(THREADS, 128 * PT_WIDE_WF_BLOCKS / THREADS) wf
     const float4* tris = nullptr;
     const RenderParams* p = nullptr;
     __shared__ uint2 sstack[SH * THREADS];
-    WideWalkT<kWideStack, SH> k;
+    WideSpill<SH, false> spill;
+    WideWalkT<kWideStack, SH, true> k;
+    k.stack.spill = spill.pairs;
     k.stack.base = sstack + threadIdx.x;
     k.stack.stride = THREADS;
     k.cur = kWideDone;
@@ -223,9 +225,10 @@ __global__ void __launch_bounds__(THREADS, 128 * PT_WIDE_WF_BLOCKS / THREADS) wf
                     const float4 o4 = SHADOW ? ws.sh_o[entry] : ws.ray_o[slot];
                     float dx, dy, dz;
                     dir(dx, dy, dz);
-                    const BinaryRay ray{o4.x, o4.y, o4.z, dx, dy, dz, SHADOW ? o4.w : __int_as_float(0x7F800000), k.any};
-                    BinaryHit b;
-                    ok = wide_binary_walk((const uint4*)p->nodes, (const float4*)p->tris, p->num_nodes, &ray, &b);
+                    auto& rest = spill.rest;
+                    rest.ray = BinaryRay{o4.x, o4.y, o4.z, dx, dy, dz, SHADOW ? o4.w : __int_as_float(0x7F800000), k.any};
+                    ok = wide_binary_walk((const uint4*)p->nodes, (const float4*)p->tris, p->num_nodes, &rest.ray, &rest.hit, rest.stack);
+                    const BinaryHit b = rest.hit;
                     k.prim = b.prim; k.leaf = b.leaf;
                     k.u = b.u; k.v = b.v; k.w = b.w;
                 }
@@ -662,7 +665,9 @@ __global__ void __launch_bounds__(128, TL ? PT_WIDE_TL_BLOCKS : PT_WIDE_PATH_BLO
     bool two = false, inside = true;  // the lane's scene is two-level; its walk is in an instance (or that is none)
     bool sure = true;                 // a face was accepted in that instance: its box has passed
     const ColdLane cold{sfield + threadIdx.x};
-    WideWalkT<kWideStack, SH> k;
+    WideSpill<SH, TL> spill;
+    WideWalkT<kWideStack, SH, true> k;
+    k.stack.spill = spill.pairs;
     k.stack.base = sstack + threadIdx.x;
     k.stack.stride = 128;
     k.cur = kWideDone;
@@ -884,16 +889,20 @@ __global__ void __launch_bounds__(128, TL ? PT_WIDE_TL_BLOCKS : PT_WIDE_PATH_BLO
             const bool shadow = (state & kRayMask) == kOnShadow;
             const F3 o = cold.f3at(kPo), d = cold.f3at(shadow ? kPw : kPd);
             const RenderParams* p = items[cold.u(kPitem)].params;
-            const BinaryRay ray{o.x, o.y, o.z, d.x, d.y, d.z, shadow ? cold.f(kPt) : bitsf(0x7F800000u), shadow};
-            BinaryHit b;
-            if (TL && two) {
-                const TwoLevelView view = two_level_view(*p);
-                uint32_t inst = 0;
-                ok = wide_two_level_walk(&view, &ray, &b, &inst);
-                cold.set(kPhitInst, inst);
-            } else {
-                ok = wide_binary_walk((const uint4*)p->nodes, (const float4*)p->tris, p->num_nodes, &ray, &b);
+            auto& rest = spill.rest;
+            rest.ray = BinaryRay{o.x, o.y, o.z, d.x, d.y, d.z, shadow ? cold.f(kPt) : bitsf(0x7F800000u), shadow};
+            bool walked = false;
+            if constexpr (TL) {
+                if (two) {
+                    const TwoLevelView view = two_level_view(*p);
+                    uint32_t inst = 0;
+                    ok = wide_two_level_walk(&view, &rest.ray, &rest.hit, &inst, rest.stack);
+                    cold.set(kPhitInst, inst);
+                    walked = true;
+                }
             }
+            if (!walked) ok = wide_binary_walk((const uint4*)p->nodes, (const float4*)p->tris, p->num_nodes, &rest.ray, &rest.hit, rest.stack);
+            const BinaryHit b = rest.hit;
             k.prim = b.prim; k.leaf = b.leaf;
             k.u = b.u; k.v = b.v; k.w = b.w;
             k.binary = false;

@@ -38,7 +38,8 @@ constexpr uint32_t kWideIndex = 0x0FFFFFFFu;
 constexpr uint32_t kWideBig = 7u;             // leaf of more than 6 faces: the index names its binary node
 constexpr uint32_t kWideEmpty = kWideLeaf;    // empty slot: a leaf without faces (visited or entered by no walk)
 constexpr uint32_t kWideDone = 0xFFFFFFFFu;   // no slot's reference: WideWalkT::cur at the end of a walk
-constexpr int kWideStack = 100;               // 1 + 3 entries a level, 32 levels of two binary ones each
+constexpr int kWideStack = 96;                // 3 entries a level of records, at most 31 levels, a fourth on the
+                                              // last, and an exit marker (trees of PT_TRAVERSAL_STACK - 2 levels)
 
 // Slot s of axis k covers [org[k] + step * (1 + q_lo 2^-15), org[k] + step * (1 + q_hi 2^-15)], where
 // step (a power of two) is 2^15 grid steps: the planes' bytes go into the mantissa of a number in [1,
@@ -171,12 +172,20 @@ PT_HD bool wide_make(const uint4* nodes, const uint32_t* wide_of, uint32_t ni, f
 // ---- the walk ---------------------------------------------------------------------------------------
 
 // Stack of one lane's walk: {near, reference} pairs, the first SH in shared memory (pair i of the lane at
-// base[i * stride], consecutive lanes on consecutive pairs), the rest in local memory.
-template <int CAP, int SH>
-struct WideStack {
+// base[i * stride], consecutive lanes on consecutive pairs), the rest in local memory: here, or LENT by
+// the kernel (WideSpill::pairs).
+template <int N, bool LENT>
+struct WidePairs {
+    uint2 spill[N];
+};
+template <int N>
+struct WidePairs<N, true> {
+    uint2* spill;
+};
+template <int CAP, int SH, bool LENT>
+struct WideStack : WidePairs<CAP - SH, LENT> {
     uint2* base;
     uint32_t stride;
-    uint2 spill[CAP - SH];
     PT_HD void put(int i, uint32_t ref, float near_t) {
         uint2 v;
         v.x = fbits(near_t);
@@ -184,17 +193,17 @@ struct WideStack {
         if constexpr (SH > 0) {
             if (i < SH) { base[i * stride] = v; return; }
         }
-        spill[i - SH] = v;
+        this->spill[i - SH] = v;
     }
     PT_HD uint2 get(int i) const {
         if constexpr (SH > 0) {
             if (i < SH) return base[i * stride];
         }
-        return spill[i - SH];
+        return this->spill[i - SH];
     }
 };
 
-template <int CAP = kWideStack, int SH = 0>
+template <int CAP = kWideStack, int SH = 0, bool LENT = false>
 struct WideWalkT {
     RayState r;         // ix, iy, iz cut at kWideSlope times the least of them (cut: some was)
     float min_t;
@@ -204,7 +213,7 @@ struct WideWalkT {
     bool binary;        // the hit is the binary walk's to find (unsuitable ray, or MinT rose)
     uint32_t cur;       // what comes next: a record, a leaf (kWideLeaf), or kWideDone
     int sp;
-    WideStack<CAP, SH> stack;
+    WideStack<CAP, SH, LENT> stack;
 };
 
 // Cuts 1/d of a ray (r set up for direction d) for a tree of the given size; false for the rays that the
@@ -234,8 +243,8 @@ PT_HD bool wide_cut(RayState& r, bool& cut, float size) {
 // Starts the walk of the ray in k.r at record 0.  Rays that wide_cut refused (fits), and those with a
 // negative or NaN far bound (the binary walk's test of an origin strictly inside a box cannot matter
 // for the others), are done at once, `binary` set.
-template <int CAP, int SH>
-PT_HD void wide_start(WideWalkT<CAP, SH>& k, float tmax, bool any, bool fits) {
+template <int CAP, int SH, bool LENT>
+PT_HD void wide_start(WideWalkT<CAP, SH, LENT>& k, float tmax, bool any, bool fits) {
     fits = fits && tmax >= 0.f;
     k.min_t = tmax;
     k.prim = kPrimNone;
@@ -247,8 +256,8 @@ PT_HD void wide_start(WideWalkT<CAP, SH>& k, float tmax, bool any, bool fits) {
     k.sp = 0;
 }
 
-template <int CAP, int SH>
-PT_HD void wide_begin(WideWalkT<CAP, SH>& k, float ox, float oy, float oz, float dx, float dy, float dz, float tmax, bool any,
+template <int CAP, int SH, bool LENT>
+PT_HD void wide_begin(WideWalkT<CAP, SH, LENT>& k, float ox, float oy, float oz, float dx, float dy, float dz, float tmax, bool any,
                       float size) {
     ray_setup(k.r, ox, oy, oz, dx, dy, dz);
     const bool fits = wide_cut(k.r, k.cut, size);
@@ -268,17 +277,21 @@ PT_HD uint32_t wide_take(uint32_t left, uint32_t warps, uint32_t chunk) {
     return left > 8 * share ? 2 * chunk : left > 4 * share ? chunk : left > 2 * share ? 32u : kWideFew;
 }
 
-// The binary walk of a whole ray, out of line: the hit in *out, false on a guard failure.  Nodes come in
-// two 128-bit loads: ptxas 12.9 does not compile the 256-bit load in a function that is not inlined.
+// The binary walk of a whole ray, out of line: the hit in *out, false on a guard failure; stack has room for
+// kStackCap entries.  Nodes come in two 128-bit loads: ptxas 12.9 does not compile the 256-bit load in a
+// function that is not inlined.
 struct BinaryRay { float ox, oy, oz, dx, dy, dz, tmax; bool any; };
 struct BinaryHit { float t, u, v, w; uint32_t prim, leaf; };
-PT_COLD bool wide_binary_walk(const uint4* nodes, const float4* tris, uint32_t num_nodes, const BinaryRay* ray, BinaryHit* out) {
-    RayWalkT<kStackCap, 0> k;
+PT_COLD bool wide_binary_walk(const uint4* nodes, const float4* tris, uint32_t num_nodes, const BinaryRay* ray, BinaryHit* out,
+                              uint32_t* stack) {
+    RayWalkT<1, 0> k;
     walk_begin(k, ray->ox, ray->oy, ray->oz, ray->dx, ray->dy, ray->dz, ray->tmax, ray->any, false);
     const bool inside = needs_inside_test(k.r, ray->tmax);
     bool ok = true;
-    while (ok && !k.done && k.sp > 0) {
-        const uint32_t ni = k.stack.get(--k.sp);
+    int sp = 0;
+    stack[sp++] = 0;
+    while (ok && !k.done && sp > 0) {
+        const uint32_t ni = stack[--sp];
         if (ni >= num_nodes) { ok = false; break; }
         const uint4 a = ldg(nodes + 2 * (size_t)ni), b = ldg(nodes + 2 * (size_t)ni + 1);
         if (!box_hits(k.r, bitsf(a.x), bitsf(a.y), bitsf(a.z), bitsf(a.w), bitsf(b.x), bitsf(b.y), k.min_t, inside)) continue;
@@ -287,19 +300,38 @@ PT_COLD bool wide_binary_walk(const uint4* nodes, const float4* tris, uint32_t n
             walk_leaf<false>(k, tris, b.z, nf);
             continue;
         }
+        if (sp + 2 > kStackCap) { ok = false; break; }
         const bool neg = neg_on(k.r, b.w >> 16);
-        ok = k.stack.put2(k.sp, neg ? ni + 1 : ni + b.z, neg ? ni + b.z : ni + 1);
-        k.sp += 2;
+        stack[sp++] = neg ? ni + 1 : ni + b.z;
+        stack[sp++] = neg ? ni + b.z : ni + 1;
     }
     out->t = k.min_t;
     out->u = k.u; out->v = k.v; out->w = k.w;
     out->prim = k.prim; out->leaf = k.leaf;
     return ok;
 }
+PT_HD bool wide_binary_walk(const uint4* nodes, const float4* tris, uint32_t num_nodes, const BinaryRay* ray, BinaryHit* out) {
+    uint32_t stack[kStackCap];
+    return wide_binary_walk(nodes, tris, num_nodes, ray, out, stack);
+}
+
+// A kernel's local memory for one lane's walks.  A ray that goes to the binary walk has ended its own, so that
+// walk's ray, hit and stacks (TL: of both levels) lie where its stack was.  Without that, and with 100 pairs,
+// the kernels' frames were 1184 to 1536 bytes; above 1024 the context's local memory grows by 46 to 98
+// MiB at the first launch, also that of a call that is to allocate none (pt_render_noalloc).
+template <int SH, bool TL>
+union WideSpill {
+    uint2 pairs[kWideStack - SH];
+    struct {
+        BinaryRay ray;
+        BinaryHit hit;
+        uint32_t stack[kStackCap + (TL ? kTopStackCap : 0)];
+    } rest;
+};
 
 // The next entry that MinT does not rule out (or kWideDone), into k.cur.
-template <int CAP, int SH>
-PT_HD void wide_pop(WideWalkT<CAP, SH>& k) {
+template <int CAP, int SH, bool LENT>
+PT_HD void wide_pop(WideWalkT<CAP, SH, LENT>& k) {
     k.cur = kWideDone;
     while (k.sp > 0) {
         const uint2 e = k.stack.get(--k.sp);
@@ -338,8 +370,8 @@ PT_HD void wide_fma2(float a0, float a1, float b0, float b1, float c0, float c1,
 // the first, near takes B - 2^-21 |B| and far B + 2^-20 |B|, which also holds the factor 1 + 2 gamma_3
 // = 1 + 3 * 2^-23 that the exact test puts on far; far's A has that factor too.  Nothing overflows:
 // |A| <= 2^9 size * 2^50 least, |B| <= 2^22 size * 2^50 least, and size * least <= 2^50.
-template <int CAP, int SH>
-PT_HD bool wide_visit(WideWalkT<CAP, SH>& k, const WideNode* __restrict__ wide) {
+template <int CAP, int SH, bool LENT>
+PT_HD bool wide_visit(WideWalkT<CAP, SH, LENT>& k, const WideNode* __restrict__ wide) {
     const uint4* p = (const uint4*)(wide + k.cur);
     uint4 w0, w1, w2, w3;
     ldg_node(p, w0, w1);
@@ -429,8 +461,8 @@ PT_HD bool wide_leaf_passes(const K& k, float4 q0, float4 q1, float4 q2, const N
 // here (an any-hit ray accepted a face, or MinT rose and `binary` is set).  `nodes` gives the binary nodes,
 // which only large leaves and boxes to be tested exactly need, `face_base` the face record of the tree's first
 // face (large leaves).  Returns whether a face was accepted.
-template <int CAP, int SH, class Nodes, class Dir, class Base>
-PT_HD bool wide_faces(WideWalkT<CAP, SH>& k, const float4* __restrict__ tris, const Nodes& nodes, const Dir& dir, const Base& face_base) {
+template <int CAP, int SH, bool LENT, class Nodes, class Dir, class Base>
+PT_HD bool wide_faces(WideWalkT<CAP, SH, LENT>& k, const float4* __restrict__ tris, const Nodes& nodes, const Dir& dir, const Base& face_base) {
     uint32_t at = k.cur & kWideIndex, n = (k.cur >> 28) & 7u;
     if (n == kWideBig) {
         uint4 a, b;
@@ -489,8 +521,8 @@ PT_HD void wide_to_object(const DeviceInstance* inst, V& o, V& d) {
 // A lane at an exit marker or a top-level leaf: leaves its instance (inside), if it is in one, or passes over
 // an empty slot.  Returns whether k.cur is then an instance to enter; else it is a top-level record, another
 // empty slot (for the next crossing), or kWideDone.
-template <int CAP, int SH>
-PT_HD bool wide_cross(WideWalkT<CAP, SH>& k, bool& inside) {
+template <int CAP, int SH, bool LENT>
+PT_HD bool wide_cross(WideWalkT<CAP, SH, LENT>& k, bool& inside) {
     if (k.cur == kWideExit || k.cur == kWideEmpty) {
         inside = false;
         wide_pop(k);
@@ -500,8 +532,8 @@ PT_HD bool wide_cross(WideWalkT<CAP, SH>& k, bool& inside) {
 
 // Enters the instance whose tree starts at record root, with its object ray in k.r.  False when that ray is
 // none for the records (wide_cut's fits; done and `binary` set) or the stack is full (done set).
-template <int CAP, int SH>
-PT_HD bool wide_enter(WideWalkT<CAP, SH>& k, uint32_t root, bool fits) {
+template <int CAP, int SH, bool LENT>
+PT_HD bool wide_enter(WideWalkT<CAP, SH, LENT>& k, uint32_t root, bool fits) {
     if (!fits || k.sp >= CAP) {
         k.done = true;
         k.binary = !fits;
@@ -524,15 +556,19 @@ PT_HD bool wide_instance_passes(const WideNode* __restrict__ wide, const uint4* 
 }
 
 // The whole ray by traverse_two_level, out of line: the hit in *out, its instance in *inst; false on a guard
-// failure.
-PT_COLD bool wide_two_level_walk(const TwoLevelView* v, const BinaryRay* ray, BinaryHit* out, uint32_t* inst) {
-    const TwoLevelHit h = traverse_two_level<false, kStackCap, true>(*v, ray->ox, ray->oy, ray->oz, ray->dx, ray->dy, ray->dz, ray->tmax,
-                                                                     ray->any);
+// failure; stack has room for kTopStackCap + kStackCap entries.
+PT_COLD bool wide_two_level_walk(const TwoLevelView* v, const BinaryRay* ray, BinaryHit* out, uint32_t* inst, uint32_t* stack) {
+    const TwoLevelHit h = traverse_two_level_on<false, kStackCap, true>(stack, stack + kTopStackCap, *v, ray->ox, ray->oy, ray->oz, ray->dx,
+                                                                        ray->dy, ray->dz, ray->tmax, ray->any);
     out->t = h.r.t;
     out->u = h.r.u; out->v = h.r.v; out->w = h.r.w;
     out->prim = h.r.prim; out->leaf = h.r.leaf;
     *inst = h.inst;
     return !h.r.overflow;
+}
+PT_HD bool wide_two_level_walk(const TwoLevelView* v, const BinaryRay* ray, BinaryHit* out, uint32_t* inst) {
+    uint32_t stack[kTopStackCap + kStackCap];
+    return wide_two_level_walk(v, ray, out, inst, stack);
 }
 
 }  // namespace pt
