@@ -259,8 +259,8 @@ PT_HD uint32_t path_fused(const RenderParams& p, uint64_t path, float* out, uint
 // ---- fused pipeline over four-wide records ------------------------------------------------------
 
 // One ray's whole walk (k set up by wide_begin for direction d).  False on a guard failure.
-template <class K, class Spill>
-PT_HD bool wide_trace(K& k, Spill& spill, const RenderParams& p, const F3& d, float tmax) {
+template <class K>
+PT_HD bool wide_trace(K& k, const RenderParams& p, const F3& d, float tmax) {
     auto dir = [&](float& x, float& y, float& z) { x = d.x; y = d.y; z = d.z; };
     while (k.cur != kWideDone) {
         while (!(k.cur & kWideLeaf)) {
@@ -273,10 +273,9 @@ PT_HD bool wide_trace(K& k, Spill& spill, const RenderParams& p, const F3& d, fl
         wide_pop(k);
     }
     if (!k.binary) return true;
-    auto& rest = spill.rest;
-    rest.ray = BinaryRay{k.r.ox, k.r.oy, k.r.oz, d.x, d.y, d.z, tmax, k.any};
-    const bool ok = wide_binary_walk((const uint4*)p.nodes, (const float4*)p.tris, p.num_nodes, &rest.ray, &rest.hit, rest.stack);
-    const BinaryHit b = rest.hit;
+    const BinaryRay ray{k.r.ox, k.r.oy, k.r.oz, d.x, d.y, d.z, tmax, k.any};
+    BinaryHit b;
+    const bool ok = wide_binary_walk((const uint4*)p.nodes, (const float4*)p.tris, p.num_nodes, &ray, &b, (uint32_t*)k.stack.spill);
     k.prim = b.prim; k.leaf = b.leaf;
     k.u = b.u; k.v = b.v; k.w = b.w;
     return ok;
@@ -294,9 +293,9 @@ PT_HD uint32_t path_wide(const RenderParams& p, uint64_t path, float* out, uint3
     s.L = f3(0.f, 0.f, 0.f);
     s.bounces = 0;
     s.last_lambert = 0;
-    WideSpill<SH, false> spill;
-    WideWalkT<kWideStack, SH, true> k;
-    k.stack.spill = spill.pairs;
+    // Its own stack, which the binary walk then takes: with a lent one (WideSpill) a 1280x720x8 frame of 1.6 M
+    // faces takes 16.8 ms instead of 10.4, one of 20 k box faces 7.9 instead of 4.6.
+    WideWalkT<kWideStack, SH> k;
     k.stack.base = stack;
     k.stack.stride = stride;
     ShadowReq sh;
@@ -307,7 +306,7 @@ PT_HD uint32_t path_wide(const RenderParams& p, uint64_t path, float* out, uint3
         const F3 d = shadow ? sh.wi : s.d;
         const float tmax = shadow ? sh.tmax : inf;
         wide_begin(k, s.o.x, s.o.y, s.o.z, d.x, d.y, d.z, tmax, shadow, p.wide_size);
-        const bool ok = wide_trace(k, spill, p, d, tmax);
+        const bool ok = wide_trace(k, p, d, tmax);
         ++rays;
         if (!ok) { raise_flag(p.err); break; }
         if (shadow) {
