@@ -167,8 +167,8 @@ int fail(int code, const std::string& msg) {
 // staging buffers and its own stream -- rays into pinned memory, to the device, kernel, hits back, out of
 // pinned memory.  Copying into and out of the staging buffers is what such a call spends its time on
 // (one thread: 5.9 ms for 1 M rays on a host of 16 threads, of which the kernel takes 0.3), so it is what
-// runs in parallel, and one worker's copies overlap another's transfers and kernel: 2.0 ms with eight;
-// 16 M rays 76.9 -> 24 ms; 70 k rays 0.53 -> 0.49.
+// runs in parallel, and one worker's copies overlap another's transfers and kernel: 1.9 ms with eight;
+// 100 k rays 0.47 -> 0.35 to 0.43, 300 k 1.18 -> 0.63.
 static int trace_pageable(pt_scene* s, const TraceArgs& common, const pt_ray* rays, uint64_t n, pt_hit* hits, bool pin_rays,
                           bool pin_hits, cudaEvent_t dep, int workers) {
     constexpr uint64_t slot_rays = kSlots * kChunkRays / kWorkers;

@@ -12,7 +12,10 @@
 namespace pt {
 
 constexpr int kWorkers = 8;
-constexpr uint64_t kPageableRays = 1 << 16;  // below, the threads cost more than they bring
+// Below, the threads cost more than they bring.  Pipelined copies / workers on a B200's host of 16 threads, medians
+// of several runs (ms): 65,536 rays 0.35 / 0.32 to 0.44, 80,000 0.40 / 0.47 to 0.51, 90,000 0.43 / 0.36 to 0.54
+// (two workers), 98,304 0.46 / 0.34 to 0.43 (three), 131,072 0.58 / 0.38 (four).
+constexpr uint64_t kPageableRays = 3 << 15;
 
 // Whether this process may run on one processor only.
 inline bool one_processor() {

@@ -51,14 +51,15 @@ static void threads() {
 // One worker (the pipelined copies) for small calls and on one processor; else two at least.
 static void counts() {
     using pt::pageable_workers;
-    for (uint64_t n : {0ull, 1ull, (1ull << 16) - 1, 1ull << 16, 1ull << 24})
+    for (uint64_t n : {0ull, 1ull, (1ull << 16) - 1, 1ull << 16, (3ull << 15) - 1, 3ull << 15, 1ull << 24})
         for (unsigned t : {0u, 1u, 2u, 16u, 256u}) {
             CHECK(pageable_workers(n, t, true) == 1);
-            CHECK((pageable_workers(n, t, false) > 1) == (n >= 1 << 16));
+            CHECK((pageable_workers(n, t, false) > 1) == (n >= 3 << 15));
         }
     for (unsigned t : {0u, 1u, 2u, 3u, 4u, 5u}) CHECK(pageable_workers(1u << 24, t, false) == 2);
     CHECK(pageable_workers(1u << 24, 16, false) == 8 && pageable_workers(~0ull, 256, false) == 8);
-    CHECK(pageable_workers(1u << 16, 64, false) == 2 && pageable_workers(3u << 15, 64, false) == 3);
+    CHECK(pageable_workers(3u << 15, 64, false) == 3 && pageable_workers((4u << 15) - 1, 64, false) == 3);
+    CHECK(pageable_workers(4u << 15, 64, false) == 4);
 }
 
 int main(int argc, char** argv) {
