@@ -399,7 +399,7 @@ typedef struct pt_batch_item {
  *                          a shade kernel appending to ray / shadow queues, a persistent shadow
  *                          kernel (wave_pixels: paths per wave).  Waves of few paths (131,072 a
  *                          bounce at most) run as PT_PIPELINE_PATHS when all scenes have
- *                          four-wide records; waves above 2^24 paths walk binary nodes.
+ *                          four-wide records.
  *   PT_PIPELINE_PATHS:     waves of paths of all renders as in PT_PIPELINE_WAVEFRONT, but one
  *                          persistent kernel runs whole paths (wave_pixels: paths per wave). */
 #define PT_PIPELINE_FUSED     0u

@@ -131,10 +131,3 @@
 #ifndef PT_WIDE_WAVE_PATHS
 #define PT_WIDE_WAVE_PATHS (1u << 17)
 #endif
-// Paths up to which a wave's extend and shadow kernels walk the records.  In longer waves all warps stay
-// busy with alike rays, and on box scenes the binary walk's 64 registers gain more than the records do: 256
-// uneven renders in waves of 33.5 M paths 1043 ms against 1073, four scenes of 20 k box faces 65.0 / 66.0
-// (of instanced spheres 16.1 / 12.9, which the path pipeline renders faster still); at 16.8 M 33.3 / 33.1.
-#ifndef PT_WIDE_WAVE_MOST
-#define PT_WIDE_WAVE_MOST (1u << 24)
-#endif

@@ -1183,9 +1183,7 @@ cudaError_t trace_stage(const WfItem* items, const WfState& ws, const uint32_t* 
 // Camera rays of the wave's slots, then per bounce: extend, shade (queue the next rays and the
 // shadow rays), shadow; finally the clamped radiance of every slot.
 cudaError_t bounce_stages(const WfItem* d_items, const WfSegment* d_segments, const WfWave& w, const WfState& ws,
-                          const WfTuning& tuning, unsigned long long* rays_traced, cudaStream_t s) {
-    WfTuning t = tuning;
-    t.wide = t.wide && w.count <= PT_WIDE_WAVE_MOST;
+                          const WfTuning& t, unsigned long long* rays_traced, cudaStream_t s) {
     const uint32_t blocks = (w.count + 127) / 128;
     wf_init_kernel<<<blocks, 128, 0, s>>>(d_items, d_segments + w.seg_begin, w.seg_count, w.count, ws);
     cudaError_t e = cudaGetLastError();

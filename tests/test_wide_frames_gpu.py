@@ -67,7 +67,8 @@ def test_batches_match_the_binary_walk(cuda_device, pipeline, threads):
         b.close()
 
 
-@pytest.mark.parametrize("width, depth, spp, wave", [(512, 2, 3, 0), (513, 2, 3, 0), (515, 0, 3, 256 * 600), (512, 0, 128, 1 << 25)])
+@pytest.mark.parametrize("width, depth, spp, wave", [(512, 2, 3, 0), (513, 2, 3, 0), (515, 0, 3, 256 * 600), (512, 0, 128, 1 << 25),
+                                                     (512, 0, 129, 1 << 25)])
 def test_waves_match_the_binary_walk(cuda_device, width, depth, spp, wave):
     """Waves that run as whole paths, bounce by bounce over records, and both in one batch."""
     wide, binary = both("boxes")
