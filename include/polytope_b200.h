@@ -407,8 +407,12 @@ typedef struct pt_batch_item {
 #define PT_PIPELINE_PATHS     2u
 typedef struct pt_batch_tuning {
     uint64_t wave_pixels;             /* work per launch / wave; 0 = automatic                    */
-    uint32_t threads_per_block;       /* 64, 128 or 256                                           */
-    uint32_t stack_depth;             /* traversal stack entries (24/32/48/64; 0 = smallest fit)   */
+    uint32_t threads_per_block;       /* 64, 128 or 256 (the fused kernel and the per-bounce ray
+                                       * kernels; the whole-path kernels have blocks of 128)      */
+    uint32_t stack_depth;             /* traversal stack entries (24/32/48/64; 0 = smallest fit) of
+                                       * walks over binary nodes: the fused kernel, and waves with a
+                                       * scene without four-wide records.  Checked for all scenes,
+                                       * without effect on walks over records                     */
     uint32_t queue_chunk;             /* pixels or rays a warp takes per fetch (multiple of 32)   */
     uint32_t pipeline;                /* PT_PIPELINE_*                                            */
 } pt_batch_tuning;

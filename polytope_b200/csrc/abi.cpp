@@ -410,7 +410,8 @@ int prepare_scene_host(const pt_scene_desc* desc, HostScene& h) {
     h.num_prims = w.num_prims;
     h.prim_base = w.prim_base;
     h.nodes.swap(t.nodes);
-    // faces in leaf order, 48 B each: {v0.xyz v1.x}{v1.yz v2.xy}{v2.z prim mesh 0}
+    // faces in leaf order, 48 B each: {v0.xyz v1.x}{v1.yz v2.xy}{v2.z prim mesh, leaf}: the last word is 0 until the
+    // records are made, then the face's leaf node (wide_mark_leaf)
     h.tris.assign(12 * (size_t)w.num_prims, 0.f);
     for (size_t i = 0; i < w.num_prims; ++i) {
         const uint32_t m = t.leaf_pairs[2 * i], f = t.leaf_pairs[2 * i + 1];

@@ -44,9 +44,10 @@
 // Walks over four-wide records: resident blocks of 128 threads a SM, lanes at a leaf before faces are
 // tested, ended lanes before new rays are taken, and visits a lane makes between votes.  Measured on a
 // B200 (us; 16.7 M rays on 1.3 M faces / 1 M rays on 100 k box faces / 1 M occlusion rays on 330 k
-// faces): 4 visits 5190 / 427 / 562, 1: 5450 / 464 / 578, 2: 5357 / 438 / 568, 8: 5387 / 438 / 605; at 4
-// visits, 6 blocks (80 registers, spills) 5484 / 437 / 586, 4 blocks 5696 / 447 / 552; leaf batch 12
-// 5280 / 427 / 554, 20 5328 / 441 / 590.
+// faces): 4 visits 4926 / 500 / 483, 1: 5293 / 523 / 511, 2: 5126 / 513 / 493, 8: 5082 / 520 / 517; at 4
+// visits, 4 blocks 5778 / 566 / 516, 6 blocks (80 registers) 4590 / 478 / 477, but 37.2 against 36.6 on 1 k
+// rays (chosen when the walk spilled there, 5484 against 5190 on the first); leaf batch 12 5039 / 498 /
+// 478, 20 5011 / 514 / 497.
 #ifndef PT_WIDE_BLOCKS
 #define PT_WIDE_BLOCKS 5
 #endif
@@ -60,12 +61,11 @@
 #define PT_WIDE_STEPS 4
 #endif
 // A warp that has no more rays to take is as slow as its slowest lane: there fewer lanes wait for faces to
-// be tested, and a lane may test a second leaf at once.  1 k rays 26.9 -> 25.6 us, 100 k on box faces 97 ->
-// 95, 1 M occlusion rays 565 -> 517, 16.7 M rays 5187 -> 5128 (the path kernel's 1920x1080x16 frame, a
-// second leaf only: 9.24 -> 9.12 ms).  With all rays a second leaf costs 7 % on 16.7 M.  A batch of 16 there
-// gives 25.7 / 92.5 / 540 / 5119, of 4 27.4 / 95.7 / 505 / 5161; four leaves 25.7 / 93.1 / 543 / 5135; 8
-// visits between votes 25.5 / 91.5 / 543 / 5147 at 16.  Two-level queries are 1 % slower with it and keep
-// the constants above.
+// be tested, and a lane may test a second leaf at once.  1 k rays 36.6 us, 100 k on box faces 94.7, 1 M
+// occlusion rays 483, 16.7 M rays 4926; a batch of 16 there, as elsewhere, gives 48.5 / 97.0 / 499 / 4921, of 4
+// 36.5 / 95.0 / 467 / 4930; one leaf 36.9 / 92.6 / 491 / 4936, four 39.1 / 95.9 / 483 / 4930.  (With all rays,
+// and before the frames were halved, a second leaf cost 7 % on 16.7 M; two-level queries were 1 % slower with
+// these and keep the constants above.)
 #ifndef PT_WIDE_LAST_BATCH
 #define PT_WIDE_LAST_BATCH 8
 #endif
@@ -74,11 +74,12 @@
 #endif
 
 // Resident blocks of 128 and leaf batch of the extend and shadow kernels (wf_wide_kernel).  Their rays come
-// from one wave and are alike, so more warps pay although the walk spills (72 registers, about 150 B).
-// Measured on a B200 (ms, four renders of depth 6; scenes of 500 k box faces / 20 k box faces / instanced
-// spheres, 33.5 M paths in one wave; the binary walk's kernel 61.0 / 65.0 / 16.1): 7 blocks and 12 59.5 /
-// 66.0 / 12.9, 6 and 12 60.5 / 67.0 / 13.1, 8 and 12 60.6 / 66.6 / 13.0, 5 and 16 65.3 / 71.0 / 13.6; with
-// waves of 4.2 M paths (binary 9.39 / 9.89 / 4.75) 8.68 / 9.30 / 2.93, 5 and 16 9.20 / 9.73 / 2.92.
+// from one wave and are alike, so more warps pay although the walk spills (72 registers, about 100 B;
+// launched with 256 threads they are three blocks of those a SM, 80 registers, and as fast).  Measured on
+// a B200 (ms, four renders of depth 6; scenes of 500 k box faces / 20 k box faces / instanced spheres,
+// 33.5 M paths in one wave; the binary walk's kernel 52.2 / 74.1 / 38.5): 7 blocks and 12 46.1 / 69.0 /
+// 29.4, 6 and 12 46.5 / 69.9 / 30.0, 8 and 12 47.5 / 69.5 / 29.3, 5 and 16 48.6 / 72.1 / 30.9; with waves of
+// 4.2 M paths 6.50 / 9.55 / 5.25, 5 and 16 6.68 / 9.85 / 5.32.
 #ifndef PT_WIDE_WF_BLOCKS
 #define PT_WIDE_WF_BLOCKS 7
 #endif
@@ -88,11 +89,10 @@
 
 // The same for the persistent path kernel (wf_wide_path_kernel), with the lanes that must have a ray to
 // end or start, or a hit to shade, before those steps run.  Measured on a B200 (ms; 1920x1080x16 frame
-// of 3.9 M faces / 641x479x4 frame of 20 k box faces / 24 served requests), before the binary walk's
-// kernel and after: 12.9 / 3.35 / 9.0 -> 9.4 / 2.7 / 6.1 (9.1 / 2.5 / 5.9 with the last paths handed out in
-// small lots, wide_take).  One visit between votes 9.5 / 3.0 / 6.5; 4 blocks
-// 10.2 / 2.85 / 6.2, 6 blocks 9.4 / 2.7 / 6.1 (one visit: 11.1 / 3.3 / 7.1); turns from 4 or 16 lanes on
-// within 2 %, shading from 10 or 24 lanes on 3 to 7 % slower on the first.
+// of 3.9 M faces / 641x479x4 frame of 20 k box faces / 24 served requests): 8.34 / 2.39 / 6.1 (the binary
+// walk's kernel about 1.4 times that).  One visit between votes 8.77 / 2.68 / 6.55; 4 blocks 9.22 / 2.54 /
+// 6.41, 6 blocks 8.60 / 2.55 / 6.44; turns from 4 lanes on 8.52 / 2.44 / 6.28, from 16 8.33 / 2.40 / 6.10 (and
+// 320x240x8 frames 5 % slower); shading from 10 lanes on 9.08 / 2.40 / 6.30, from 24 8.48 / 2.46 / 6.14.
 #ifndef PT_WIDE_PATH_BLOCKS
 #define PT_WIDE_PATH_BLOCKS 5
 #endif
@@ -112,8 +112,8 @@
 // Two-level scenes over four-wide records (queries and the persistent path kernel): resident blocks, and
 // lanes that must stand at an instance or an exit before those steps run.  Measured on a B200 (us, 1 M rays
 // on five instances of 82 k faces / ms, 1280x720x8 frame of five instances of 330 k faces through the
-// persistent kernel), over the binary trees before 633 / 14.5: 4 blocks 338 / 5.8, 3 blocks 390 / 7.6, 5
-// blocks 417 / 6.6, 6 blocks 473 / 7.5; entering from 4 or 16 lanes on within 2 %.
+// persistent kernel, 33.6 over the binary trees): 4 blocks 324 / 12.8, 3 blocks 370 / 15.0, 5 blocks 351 /
+// 13.4, 6 blocks 386 / 15.4; entering from 4 lanes on 328 / 12.9, from 16 356 / 14.1.
 #ifndef PT_WIDE_TL_BLOCKS
 #define PT_WIDE_TL_BLOCKS 4
 #endif
@@ -124,10 +124,9 @@
 // Paths per bounce up to which a wave over four-wide records runs as whole paths in the persistent path
 // kernel instead of bounce by bounce: a bounce costs six launches, each as long as its slowest ray, which
 // few paths don't cover.  Bounce by bounce / whole paths on a B200 (ms; eight scenes of 20 k faces each):
-// depth 0 (one bounce), 131 k paths 0.13 / 0.13, 524 k 0.26 / 0.27; depth 2, 131 k 0.65 / 0.48, 393 k 0.93 /
-// 0.90, 786 k 1.44 / 1.49; depth 6, 131 k 1.04 / 0.57, 917 k 2.16 / 1.95; depth 12, 131 k 3.11 / 1.24, 2.1 M
-// 7.66 / 6.89.  Scenes of 1 k faces gain more, of 500 k faces the same; far above the line the waves are
-// 8 % ahead (24 uneven renders, 24.5 against 26.3).
+// depth 0 (one bounce), 131 k paths 0.15 / 0.15, 524 k 0.26 / 0.25; depth 2, 131 k 0.54 / 0.43, 390 k 0.84 /
+// 0.80, 783 k 1.27 / 1.32; depth 6, 131 k 1.22 / 0.80, 913 k 2.70 / 2.57; depth 12, 131 k 2.07 / 1.17, 2.1 M
+// 6.69 / 6.28.  Far above the line the waves were 8 % ahead (24 uneven renders, 24.5 against 26.3).
 #ifndef PT_WIDE_WAVE_PATHS
 #define PT_WIDE_WAVE_PATHS (1u << 17)
 #endif

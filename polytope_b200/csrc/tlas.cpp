@@ -181,7 +181,7 @@ int prepare_two_level_host(const pt_scene_desc* desc, HostScene& h) {
         node_base.push_back((uint32_t)h.nodes.size());
         face_base.push_back((uint32_t)(h.tris.size() / 12));
         h.nodes.insert(h.nodes.end(), t.nodes.begin(), t.nodes.end());
-        // faces in leaf order, 48 B each: {v0.xyz v1.x}{v1.yz v2.xy}{v2.z face 0 0} (object space)
+        // faces in leaf order, 48 B each: {v0.xyz v1.x}{v1.yz v2.xy}{v2.z face 0, leaf (wide.cuh)} (object space)
         const size_t base = h.tris.size();
         h.tris.resize(base + 12 * (size_t)wo.num_prims, 0.f);
         for (size_t i = 0; i < wo.num_prims; ++i) {

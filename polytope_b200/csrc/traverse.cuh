@@ -12,7 +12,7 @@
 //
 // Data layout in HBM (all read with 128-bit non-coherent loads):
 //   nodes  32 B  {bb_min.xyz, bb_max.xyz, offset, num_faces | axis << 16}   (2 x uint4)
-//   tris   48 B  {v0.xyz v1.x}{v1.yz v2.xy}{v2.z prim mesh 0} in leaf order (3 x float4)
+//   tris   48 B  {v0.xyz v1.x}{v1.yz v2.xy}{v2.z prim mesh leaf} in leaf order (3 x float4; leaf: wide.cuh)
 //   rays   32 B  {org.xyz tmax}{dir.xyz flags}                              (2 x float4)
 //   hits   16 B  {prim t u v}                                              (1 x uint4)
 #pragma once

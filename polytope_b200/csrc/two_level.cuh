@@ -19,7 +19,7 @@ constexpr int kTopStackCap = PT_TOP_STACK;
 
 struct TwoLevelView {
     const uint4* nodes;          // every bottom-level tree, back to back
-    const float4* tris;          // their leaf-ordered object-space faces {v0 v1.x}{v1.yz v2.xy}{v2.z face 0 0}
+    const float4* tris;          // their leaf-ordered object-space faces {v0 v1.x}{v1.yz v2.xy}{v2.z face 0 leaf}
     uint32_t num_nodes;
     const uint4* top;            // top-level nodes
     uint32_t top_nodes;

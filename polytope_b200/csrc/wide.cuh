@@ -266,11 +266,12 @@ PT_HD void wide_begin(WideWalkT<CAP, SH, LENT>& k, float ox, float oy, float oz,
 
 // Rays (or paths) that a warp takes from the counter, `left` being those not handed out when it last took
 // some: twice `chunk` while there are plenty, kWideFew when each warp has little left to do, so that all end
-// together.  Against `chunk` throughout (64), on a B200: 16.7 M rays 5130 -> 5075 us, 1 M occlusion rays
-// 514 -> 484, 1 M on box faces 430 -> 420, a 641x479x4 frame 2.72 -> 2.53 ms, 24 uneven renders 25.0 ->
-// 24.5 ms.  Few of 8 or 32 from there on 482 / 493 us on the occlusion rays; few from `share` on instead of
-// twice that 518; shares of the rest (left / (2 warps)) 575, as early takers keep
-// too much.  Two-level queries are 1 % slower with it and take `chunk` throughout.
+// together.  Against `chunk` throughout (64), on a B200, with frames twice as large: 16.7 M rays 5130 -> 5075
+// us, 1 M occlusion rays 514 -> 484, 1 M on box faces 430 -> 420, a 641x479x4 frame 2.72 -> 2.53 ms, 24 uneven
+// renders 25.0 -> 24.5 ms; few from `share` on instead of twice that 518 on the occlusion rays; shares of the
+// rest (left / (2 warps)) 575, as early takers keep too much.  Few of 8 from there on: within 0.6 % of 16, but
+// a 320x240x8 frame 7 % slower; of 32: 2 to 5 % slower, that frame 16 %.  Two-level queries were 1 % slower
+// with it and take `chunk` throughout.
 constexpr uint32_t kWideFew = 16;
 PT_HD uint32_t wide_take(uint32_t left, uint32_t warps, uint32_t chunk) {
     const uint32_t share = warps * chunk;
